@@ -256,8 +256,13 @@ __device__ __forceinline__ void fill_phase(const DevState& s, int q, NbInfo* nbi
     if (t == 0) *s_next = (int)atomicAdd(&s.queue[4 * q], 1u);
     __syncthreads();
     int k = *s_next;
-    if (k < total && t < NBI_INTS)
-        reinterpret_cast<int*>(&nbis[0])[t] = __ldg(s.nbinfo + (size_t)k * NBI_STRIDE + t);
+    // an item's record (a CTA of a small block has fewer threads than it has words)
+    auto record = [&](int item, NbInfo* dst) {
+        for (int i = t; i < NBI_INTS; i += blockDim.x)
+            cp_async4(reinterpret_cast<int*>(dst) + i, s.nbinfo + (size_t)item * NBI_STRIDE + i);
+    };
+    if (k < total) record(k, &nbis[0]);
+    cp_async_wait_all();
     __syncthreads();
     int rb = 0;
     while (k < total) {
@@ -270,14 +275,13 @@ __device__ __forceinline__ void fill_phase(const DevState& s, int q, NbInfo* nbi
         if (t == 0) *s_next = (int)kn;
         __syncthreads();
         const int knext = *s_next;
-        int pre = 0;
-        if (knext < total && t < NBI_INTS) pre = __ldg(s.nbinfo + (size_t)knext * NBI_STRIDE + t);
+        if (knext < total) record(knext, &nbis[rb ^ 1]);
         if (do_fill) {
             walls(n, nbi);
             __syncthreads();
         }
         publish_ring(s, q, n);
-        if (t < NBI_INTS) reinterpret_cast<int*>(&nbis[rb ^ 1])[t] = pre;
+        cp_async_wait_all();
         __syncthreads();
         k = knext;
         rb ^= 1;
