@@ -24,7 +24,7 @@ __device__ __forceinline__ int ghost_dir(int x, int y, int nx, int ny) {
 // level-ordered fill waits for, and nf[q], the number of foreign cells
 struct NbInfo {
     int id[9], lev[9], leaf[9], c1[9];
-    int bi, bj;
+    int bi, bj, dx;
     int wait[NQUEUES];
     int nf[NQUEUES];
     // plan entries stored first: na of kinds 1 and -1, then n2 of kind 2, then
@@ -223,22 +223,25 @@ constexpr int REC_NF = (int)(offsetof(NbInfo, nf) / sizeof(int));
 constexpr int REC_NA = (int)(offsetof(NbInfo, na) / sizeof(int));
 constexpr int REC_N2 = (int)(offsetof(NbInfo, n2) / sizeof(int));
 constexpr int REC_N3 = (int)(offsetof(NbInfo, n3) / sizeof(int));
+constexpr int REC_DX = (int)(offsetof(NbInfo, dx) / sizeof(int));
 
 // what an item of fill q needs from its record: block, foreign cells, plan
-// entry classes, walls (id[3], id[4] < 0); staged in shared memory by
-// threads 0..6 (REC_WORDS words), read from there by every thread
+// entry classes, walls (id[3], id[4] < 0), cell size; staged in shared memory
+// by threads 0..7 (REC_WORDS words), read from there by every thread
 struct ItemRec {
     int n, nf, na, n2, n3;
     bool w3, w4;
+    int dx;
 };
-constexpr int REC_WORDS = 7;
-// word t of an item record: n, nf, na, n2, n3, id[3] (bottom), id[4] (top)
+constexpr int REC_WORDS = 8;
+// word t of an item record: n, nf, na, n2, n3, id[3] (bottom), id[4] (top), dx
 __device__ __forceinline__ const int* item_rec_word(const DevState& s, int c, int q, int t) {
     const int off = t == 0   ? 0
                     : t == 1 ? REC_NF + q
                     : t == 2 ? REC_NA + q
                     : t == 3 ? REC_N2 + q
                     : t == 4 ? REC_N3 + q
+                    : t == 7 ? REC_DX
                              : t - 2;
     return s.nbinfo + (size_t)c * NBI_STRIDE + off;
 }
@@ -246,7 +249,7 @@ __device__ __forceinline__ void item_rec_stage(const DevState& s, int c, int q, 
     const int t = threadIdx.x;
     if (t < REC_WORDS) dst[t] = __ldg(item_rec_word(s, c, q, t));
 }
-// the same without waiting for the loads: threads 0..6 gather the words with
+// the same without waiting for the loads: threads 0..7 gather the words with
 // cp.async and call cp_async_wait_all before the barrier that precedes the
 // first read of dst (thread 0, which copies word 0, may read it after its
 // own wait)
@@ -263,6 +266,7 @@ __device__ __forceinline__ ItemRec item_rec_of(const int* w) {
     o.n3 = w[4];
     o.w3 = w[5] < 0;
     o.w4 = w[6] < 0;
+    o.dx = w[7];
     return o;
 }
 

@@ -60,6 +60,7 @@ __device__ void load_nbinfo(const DevState& s, int n, NbInfo& r) {
     r.c1[0] = 0;
     r.bi = s.bi[n];
     r.bj = s.bj[n];
+    r.dx = s.dx[n];
     for (int q = 0; q < NQUEUES; ++q) r.wait[q] = r.nf[q] = 0;
 }
 
@@ -162,10 +163,10 @@ __global__ void __launch_bounds__(128, 8) k_build_plans(DevState s) {
                            return offc(blk, x2, y2);
                        },
                        sub);
-            plan_store(fc, fmax, j, sub);
+            plan_store(fc, fmax, j, sub, d);
             fc[10 * fmax + j] = (int)offc(nbi.id[d], xx, yy);
             for (int m = 0; m < 9; ++m) sub.src[m] = aoff[m];
-            plan_store(fa, fmax, j, sub);
+            plan_store(fa, fmax, j, sub, d);
             fa[10 * fmax + j] = (int)G.a(nbi.id[d], 1, xx, yy);
         }
         __syncthreads();
@@ -435,7 +436,7 @@ __device__ void fill_ring_c(const DevState& s, const Geo<N>& G, int k, int n, in
 // loads in flight together.
 template <int N>
 __device__ __forceinline__ void hg_copy(const DevState& s, const Geo<N>& G, const int* pl, int RG,
-                                        int e, int f, int n, double* As, bool to_mem) {
+                                        int e, int f, int n, double* As) {
     const int meta = pl[e];
     int x, y;
     ring1_xy(meta >> 8, G.nx, G.ny, x, y);
@@ -450,7 +451,7 @@ __device__ __forceinline__ void hg_copy(const DevState& s, const Geo<N>& G, cons
     for (int qq = 0; qq < 9; ++qq) v[qq] = __ldg(src + (size_t)qq * G.aplane);
 #pragma unroll
     for (int qq = 0; qq < 9; ++qq) {
-        if (to_mem) A[G.a(n, qq + 1, x, y)] = v[qq];
+        A[G.a(n, qq + 1, x, y)] = v[qq];
         if (As) As[f * 9 * G.aplane + G.a(0, qq + 1, x, y)] = v[qq];
     }
 }
@@ -458,7 +459,7 @@ __device__ __forceinline__ void hg_copy(const DevState& s, const Geo<N>& G, cons
 template <int N>
 __device__ __forceinline__ void hg_interp(const DevState& s, const Geo<N>& G, const int* pl, int RG,
                                           int e, int qq, int n, const double* Fs, double* As,
-                                          bool to_mem, bool cg) {
+                                          bool cg) {
     const int meta = pl[e];
     const int kind = plan_kind(meta);
     int x, y;
@@ -479,7 +480,7 @@ __device__ __forceinline__ void hg_interp(const DevState& s, const Geo<N>& G, co
             for (int i = 0; i < 9; ++i) g[i] = c2f_source(wd[i], Fs + (f * 9 + qq) * s.fmax, A, qo, cg);
         }
         const double v = plan_combine(meta, g);
-        if (to_mem) A[G.a(n, qq + 1, x, y)] = v;
+        A[G.a(n, qq + 1, x, y)] = v;
         if (As) As[f * 9 * G.aplane + G.a(0, qq + 1, x, y)] = v;
     }
 }
@@ -494,12 +495,12 @@ __device__ void fill_ring_hg(const DevState& s, const Geo<N>& G, int k, int n, i
     if (mode != 2)
         for (int u = threadIdx.x; u < 2 * RG; u += blockDim.x) {
             const int kind = plan_kind(__ldg(pl + u % RG));
-            if (kind == 1 || kind == -1) hg_copy<N>(s, G, pl, RG, u % RG, u / RG, n, nullptr, true);
+            if (kind == 1 || kind == -1) hg_copy<N>(s, G, pl, RG, u % RG, u / RG, n, nullptr);
         }
     for (int u = threadIdx.x; u < 9 * RG; u += blockDim.x) {
         const int kind = plan_kind(__ldg(pl + u % RG));
         if (kind >= 2 && pass_takes(mode, kind))
-            hg_interp<N>(s, G, pl, RG, u % RG, u / RG, n, Fs, nullptr, true, true);
+            hg_interp<N>(s, G, pl, RG, u % RG, u / RG, n, Fs, nullptr, true);
     }
 }
 
@@ -704,9 +705,9 @@ __device__ __forceinline__ unsigned macro_g_cell_f(const DevState& s, const Geo<
 // and the IEEE path for a cell whose flag says a quotient left its range.
 // SHH, SHG: Hb, Gb point to shared memory (else to memory)
 template <int N, bool FUSED, bool SHH, bool SHG, bool BGK = false, bool BATCH = false>
-__device__ __forceinline__ void collide_block(const DevState& s, const Geo<N>& G, int n,
+__device__ __forceinline__ void collide_block(const DevState& s, const Geo<N>& G, int n, int dx,
                                               const double* T, const double* Hb, const double* Gb) {
-    const double inv_dx = 1.0 / (double)__ldg(s.dx + n);  // dx is a power of two: exact
+    const double inv_dx = 1.0 / (double)dx;  // dx is a power of two: exact
     for (int c = threadIdx.x; c < G.nx * G.ny; c += blockDim.x)
         if (collide_cell<false, FUSED, SHH, SHG, N, BGK, BATCH>(s, G, n, c, inv_dx, T, Hb, Gb))
             collide_cell<true, FUSED, SHH, SHG, N, BGK, BATCH>(s, G, n, c, inv_dx, T, Hb, Gb);
@@ -715,9 +716,9 @@ __device__ __forceinline__ void collide_block(const DevState& s, const Geo<N>& G
 // Macroscopic_Values_g_AMR of every cell of block n; returns this thread's
 // maximum of the Err_Interface terms
 template <int N, bool SH, bool BATCH = false>
-__device__ __forceinline__ double macro_g_block(const DevState& s, const Geo<N>& G, int n,
+__device__ __forceinline__ double macro_g_block(const DevState& s, const Geo<N>& G, int n, int dx,
                                                 const double* T, const double* Gb) {
-    const double inv_dx = 1.0 / (double)__ldg(s.dx + n);
+    const double inv_dx = 1.0 / (double)dx;
     double mx = 0.0;
     for (int c = threadIdx.x; c < G.nx * G.ny; c += blockDim.x) {
         double dc;
@@ -745,10 +746,10 @@ __device__ __forceinline__ void err_reduce(const DevState& s, int n, double mx, 
 // Bounce_Back_3/4 (BC_Cell.f90:2-42): f(i,X,wall row) = f(opposite(i), Xn,
 // first row) on the walls of block n; after the ring fill and a barrier
 template <int N>
-__device__ void bounce_back(const DevState& s, const Geo<N>& G, int n, const NbInfo& nbi) {
+__device__ void bounce_back(const DevState& s, const Geo<N>& G, int n, bool w3, bool w4) {
     const int nx = G.nx, ny = G.ny;
     for (int wall = 3; wall <= 4; ++wall) {
-        if (nbi.id[wall] >= 0) continue;
+        if (!(wall == 3 ? w3 : w4)) continue;
         const int Y = (wall == 3) ? 0 : ny + 1, Yi = (wall == 3) ? 1 : ny;
         const int sgn = (wall == 3) ? 1 : -1;
         for (int idx = threadIdx.x; idx < (nx + 2) * 18; idx += blockDim.x) {
@@ -766,12 +767,136 @@ __device__ void bounce_back(const DevState& s, const Geo<N>& G, int n, const NbI
     }
 }
 
+// streaming coefficients of block n (dt/dx = 1/dx): Perfect_Shift_AMR where
+// the Courant number exceeds 0.9, else Lax-Wendroff with cA, cB, cC
+struct StreamCoef {
+    double cA, cB, cC;
+    bool shift;
+    __device__ __forceinline__ explicit StreamCoef(int dx) {
+        const double cfl = 1.0 / (double)dx;
+        shift = cfl > (double)0.9f;
+        cA = cfl / 2.0 * (1.0 + cfl);
+        cB = 1.0 - cfl * cfl;
+        cC = cfl / 2.0 * (1.0 - cfl);
+    }
+};
+
+// Which populations of a ghost cell in direction d streaming reads: of the
+// cells beside it, those that move from it into the block (digits 0-2) and,
+// for Lax-Wendroff only, the opposite ones (digits 3-5); 0: none. Three
+// (six) of the nine on a side, one (two) in a corner.
+__device__ __forceinline__ unsigned stream_pops(int d) {
+    switch (d) {
+        case 1: return 0x874962u;
+        case 2: return 0x962874u;
+        case 3: return 0x985763u;
+        case 4: return 0x763985u;
+        case 5: return 0x008006u;
+        case 6: return 0x007009u;
+        case 7: return 0x009007u;
+        default: return 0x006008u;
+    }
+}
+
+// Foreign cells of an h/g item (records fb) into Fs[field and population]
+// [slot]: the populations that streaming reads (nj digits of stream_pops).
+// Ends with a barrier when there are any (nf is block-uniform).
+template <int N>
+__device__ __forceinline__ void foreign_stream(const DevState& s, const Geo<N>& G, const int* fb,
+                                               int nf, int nj, double* Fs) {
+    if (nf == 0) return;
+    const int fmax = s.fmax;
+    for (int u = threadIdx.x; u < 2 * nj * nf; u += blockDim.x) {
+        const int j = u % nf, v = u / nf, f = v >= nj, m = f ? v - nj : v;
+        const int q = (int)(stream_pops(fb[j] >> 8) >> (4 * m)) & 15;
+        if (q)
+            Fs[(f * 9 + q - 1) * fmax + j] =
+                foreign_value(fb, fmax, j, f ? s.Ag : s.Ah, (size_t)(q - 1) * G.aplane, true);
+    }
+    __syncthreads();
+}
+
+// The ghost values that streaming reads, on the item's staged planes As
+// (plan words pl of ring length RG; foreign cells in Fs): copies per (entry,
+// field), interpolated cells per (entry, population, field). The first round
+// of both is loaded before `landed` (the wait for the planes' bulk copy) and
+// written after it, so that its latency overlaps the copy. Of the nine
+// populations of a ghost cell streaming reads three (Perfect_Shift_AMR) or
+// six (Lax-Wendroff), see stream_pops; only those are gathered. landed
+// returns false if the copy did not arrive. Ends with a barrier.
+template <int N, class W>
+__device__ __forceinline__ bool stream_ring(const DevState& s, const Geo<N>& G, const int* pl,
+                                            const ItemRec& r, int nj, const double* Fs, double* As,
+                                            W landed) {
+    const int RG = ring1_len(G.nx, G.ny), FP = 9 * G.aplane, fmax = s.fmax;
+    const int nC = 2 * r.na, nI = r.n2 + r.n3, T = blockDim.x;
+    double v[6];
+    auto load_copy = [&](int u) {
+        const int e = u % r.na, f = u / r.na, d = pl[e] >> 8;  // ring index
+        int x, y;
+        ring1_xy(d, G.nx, G.ny, x, y);
+        const unsigned p = stream_pops(ghost_dir(x, y, G.nx, G.ny));
+        const double* A = (f ? s.Ag : s.Ah) + (unsigned)pl[RG + e];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+            const int q = (int)(p >> (4 * m)) & 15;
+            v[m] = (m < nj && q) ? __ldg(A + (q - 1) * G.aplane) : 0.0;
+        }
+    };
+    auto store_copy = [&](int u) {
+        const int e = u % r.na, f = u / r.na;
+        int x, y;
+        ring1_xy(pl[e] >> 8, G.nx, G.ny, x, y);
+        const unsigned p = stream_pops(ghost_dir(x, y, G.nx, G.ny));
+#pragma unroll
+        for (int m = 0; m < 6; ++m) {
+            const int q = (int)(p >> (4 * m)) & 15;
+            if (m < nj && q) As[f * FP + G.a(0, q, x, y)] = v[m];
+        }
+    };
+    // interpolated value u; its place in As (-1: none)
+    auto interp = [&](int u, double& o) {
+        const int i = u % nI, w = u / nI, f = w >= nj, m = f ? w - nj : w, e = r.na + i;
+        const int meta = pl[e], kind = plan_kind(meta);
+        int x, y;
+        ring1_xy(meta >> 8, G.nx, G.ny, x, y);
+        const int q = (int)(stream_pops(ghost_dir(x, y, G.nx, G.ny)) >> (4 * m)) & 15;
+        if (!q) return -1;
+        const double* A = (f ? s.Ag : s.Ah) + (q - 1) * G.aplane;
+        const double* F = Fs + (f * 9 + q - 1) * fmax;
+        double g[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const unsigned wd = (unsigned)pl[(1 + k) * RG + e];
+            g[k] = (kind == 3 && (wd & kIndirect)) ? F[wd & ~kIndirect] : __ldg(A + wd);
+        }
+        o = plan_combine(meta, g);
+        return (int)(f * FP + G.a(0, q, x, y));
+    };
+    const int uc = threadIdx.x, ui = T - 1 - threadIdx.x, nV = 2 * nj * nI;
+    double o;
+    int at = -1;
+    if (uc < nC) load_copy(uc);
+    if (ui < nV) at = interp(ui, o);
+    if (!landed()) return false;
+    if (uc < nC) store_copy(uc);
+    if (at >= 0) As[at] = o;
+    for (int u = uc + T; u < nC; u += T) {
+        load_copy(u);
+        store_copy(u);
+    }
+    for (int u = ui + T; u < nV; u += T)
+        if ((at = interp(u, o)) >= 0) As[at] = o;
+    __syncthreads();
+    return true;
+}
+
 // The same walls on a block's h and g planes staged in shared memory (As:
-// [field][q][pool plane layout]), also written to memory. No barrier inside:
-// wall rows are written, rows 1 and ny read.
+// [field][q][pool plane layout]), also written to memory where to_mem. No
+// barrier inside: wall rows are written, rows 1 and ny read.
 template <int N>
 __device__ void bounce_back_staged(const DevState& s, const Geo<N>& G, int n, bool w3, bool w4,
-                                   double* As, bool to_mem = true) {
+                                   double* As, bool to_mem) {
     const int nx = G.nx, ny = G.ny, FP = 9 * G.aplane;
     for (int idx = threadIdx.x; idx < (nx + 2) * 36; idx += blockDim.x) {
         const int X = idx % (nx + 2), qf = (idx / (nx + 2)) % 18;
@@ -794,19 +919,6 @@ __device__ void bounce_back_staged(const DevState& s, const Geo<N>& G, int n, bo
 // LBM_Subroutines.f90:41-90) of every cell of block n into B, and
 // Macroscopic_Values_h_AMR (:193-201), from As: the block's h and g planes
 // (ring included) in shared memory, each field 9 planes in the pool layout.
-// streaming coefficients of block n (dt/dx = 1/dx): Perfect_Shift_AMR where
-// the Courant number exceeds 0.9, else Lax-Wendroff with cA, cB, cC
-struct StreamCoef {
-    double cA, cB, cC;
-    bool shift;
-    __device__ __forceinline__ StreamCoef(const DevState& s, int n) {
-        const double cfl = 1.0 / (double)__ldg(s.dx + n);
-        shift = cfl > (double)0.9f;
-        cA = cfl / 2.0 * (1.0 + cfl);
-        cB = 1.0 - cfl * cfl;
-        cC = cfl / 2.0 * (1.0 - cfl);
-    }
-};
 template <int N>
 __device__ __forceinline__ void stream_cell(const DevState& s, const Geo<N>& G, int n, const double* As,
                                             const StreamCoef& k, int x, int y) {
@@ -834,8 +946,8 @@ __device__ __forceinline__ void stream_cell(const DevState& s, const Geo<N>& G, 
     s.C[G.c(n, x, y)] = csum;
 }
 template <int N>
-__device__ void stream_block(const DevState& s, const Geo<N>& G, int n, const double* As) {
-    const StreamCoef k(s, n);
+__device__ void stream_block(const DevState& s, const Geo<N>& G, int n, const double* As,
+                             const StreamCoef& k) {
     for (int c = threadIdx.x; c < G.nx * G.ny; c += blockDim.x)
         stream_cell<N>(s, G, n, As, k, c % G.nx + 1, c / G.nx + 1);
 }
@@ -856,19 +968,20 @@ __device__ void fast_ring_c(const DevState& s, const Geo<N>& G, const int* pl, i
     __syncthreads();
 }
 
-// the same for the h/g ring on the staged planes As (if given): copies per
-// field, interpolated cells per population (both fields)
+// the same for the whole h/g ring, all nine populations, on the staged planes
+// As and in memory (the last step of a call, where the state is observed):
+// copies per field, interpolated cells per population (both fields)
 template <int N>
-__device__ void fast_ring_hg(const DevState& s, const Geo<N>& G, const int* pl, const ItemRec& r,
-                             const double* Fs, double* As, bool to_mem) {
+__device__ __forceinline__ void fast_ring_hg(const DevState& s, const Geo<N>& G, const int* pl,
+                                             const ItemRec& r, const double* Fs, double* As) {
     const int RG = ring1_len(G.nx, G.ny);
     const int nC = 2 * r.na, nI = r.n2 + r.n3;
     for (int u = threadIdx.x; u < nC + 9 * nI; u += blockDim.x) {
         if (u < nC) {
-            hg_copy<N>(s, G, pl, RG, u % r.na, u / r.na, r.n, As, to_mem);
+            hg_copy<N>(s, G, pl, RG, u % r.na, u / r.na, r.n, As);
         } else {
             const int v = u - nC;
-            hg_interp<N>(s, G, pl, RG, r.na + v % nI, v / nI, r.n, Fs, As, to_mem, false);
+            hg_interp<N>(s, G, pl, RG, r.na + v % nI, v / nI, r.n, Fs, As, false);
         }
     }
     __syncthreads();
@@ -934,15 +1047,15 @@ __device__ __forceinline__ void fill_c_body(const DevState& s, int w, int q, int
     if (collide && blockIdx.x == 0 && t == 0)
         atomicAdd(&s.cnt->updates, (unsigned long long)total * (unsigned long long)(G.nx * G.ny));
     // stage st: C tile at tiles + st*SD, then h planes (if staged), then g planes
-    auto consume = [&](int n, const double* T) {
+    auto consume = [&](int n, int dx, const double* T) {
         const double* Hs = stage_h(CONSUMER) ? T + G.cplane : s.Bh + (size_t)n * HP;
         const double* Gs = stage_g(CONSUMER) ? T + G.cplane + (stage_h(CONSUMER) ? HP : 0)
                                              : s.Bg + (size_t)n * HP;
         if (CONSUMER == CONS_MACRO_G)
-            err_reduce(s, n, macro_g_block<N, true, BATCH>(s, G, n, T, Gs), red);
+            err_reduce(s, n, macro_g_block<N, true, BATCH>(s, G, n, dx, T, Gs), red);
         else if (CONSUMER != CONS_NONE)
             collide_block<N, CONSUMER == CONS_COLLIDE_FUSED, stage_h(CONSUMER), stage_g(CONSUMER), BGK,
-                          BATCH>(s, G, n, T, Hs, Gs);
+                          BATCH>(s, G, n, dx, T, Hs, Gs);
     };
     const unsigned tb = (unsigned)G.cplane * 8, hb = (unsigned)HP * 8;
     auto copy_tile = [&](int st, int nn, int c) {  // thread 0: item c, block nn
@@ -1069,7 +1182,7 @@ __device__ __forceinline__ void fill_c_body(const DevState& s, int w, int q, int
             pend = ((int)cn < total) && !start_tile(st ^ 1, (int)cn, nn, false);
         }
         __syncwarp();  // warp 0 reconverges after thread 0's copies, before the consumer work
-        consume(n, T);
+        consume(n, fast ? r.dx : __ldg(s.dx + n), T);
         if (fast) cp_async_wait_all();  // the next item's record
         __syncthreads();
         c = s_next;
@@ -1094,10 +1207,11 @@ __global__ void __launch_bounds__(256, fill_c_min_blocks(CONSUMER))
 // Fill_Ghost_Cells_hg (Fill_Ghost_Cells_hg.f90:2-477) with Bounce_Back_3/4,
 // then streaming and Macroscopic_Values_h_AMR, one item per leaf. Each item
 // bulk-copies its block's h and g planes into shared memory. Without level
-// order (fast_fill) CTA b takes items b, b + gridDim.x, ..., fills each
-// item's ring on the staged planes (and in memory if wr), applies the walls
-// and streams; with level order the fill phase fills every leaf first and
-// consumer items come from a queue, their copy waiting for the block's flag.
+// order (fast_fill) CTA b takes items b, b + gridDim.x, ..., puts the ghost
+// values that streaming reads on the staged planes (stream_ring) and streams;
+// the whole ring goes to memory only if wr. With level order the fill phase
+// fills every leaf first and consumer items come from a queue, their copy
+// waiting for the block's flag.
 // Shared memory: mbarriers (128 bytes), h and g planes, the foreign values,
 // and without level order one item's plan words and foreign records (copied
 // once the previous item's ring is filled; a CTA's first item has its plan
@@ -1108,49 +1222,49 @@ __global__ void __launch_bounds__(256, fill_c_min_blocks(CONSUMER))
 __host__ __device__ inline size_t hg_plan_offset(size_t FP, int fmax) {
     return (128 + 8 * (2 * FP + 18 * (size_t)fmax) + 15) & ~(size_t)15;
 }
-template <int N, bool FAST>
-__device__ __forceinline__ void fill_hg_stream_body(const DevState& s, int wr, int total, int first) {
-    extern __shared__ __align__(128) unsigned char smraw[];
-    const Geo<N> G(s);
-    __shared__ NbInfo nbis[2];
-    __shared__ int s_next;
-    const int q = Q_FILLHG;
-    const int t = threadIdx.x;
-    const int FP = 9 * G.aplane;
-    unsigned long long* bar = reinterpret_cast<unsigned long long*>(smraw);
-    double* As = reinterpret_cast<double*>(smraw + 128);  // [h|g][q][pool plane layout]
-    double* Fs = As + 2 * (size_t)FP;
-    const unsigned fb = (unsigned)FP * 8;
-    auto copy_planes = [&](int nn) {  // thread 0
+// shared memory and the bulk copies of an item
+template <int N>
+struct HgStage {
+    const DevState& s;
+    const int FP, RG;
+    unsigned long long* bar;  // [planes | plan]
+    double *As, *Fs;          // [h|g][q][pool plane layout], foreign values
+    int* Ps;                  // plan words and foreign records
+    __device__ __forceinline__ HgStage(const DevState& s_, const Geo<N>& G, unsigned char* sm)
+        : s(s_), FP(9 * G.aplane), RG(ring1_len(G.nx, G.ny)) {
+        bar = reinterpret_cast<unsigned long long*>(sm);
+        As = reinterpret_cast<double*>(sm + 128);
+        Fs = As + 2 * (size_t)FP;
+        Ps = reinterpret_cast<int*>(sm + hg_plan_offset(FP, s.fmax));
+    }
+    __device__ __forceinline__ void copy_planes(int n) const {  // thread 0
+        const unsigned fb = (unsigned)FP * 8;
         fence_proxy_async_all();
         mbar_expect_tx(bar, 2 * fb);
-        bulk_g2s(As, s.Ah + (size_t)nn * FP, fb, bar);
-        bulk_g2s(As + FP, s.Ag + (size_t)nn * FP, fb, bar);
-    };
-    // without level order: plan words and foreign records of an item (Ps,
-    // mbarrier bar[1]), copied once the previous item's ring is filled
-    const int RG = ring1_len(G.nx, G.ny);
-    int* Ps = reinterpret_cast<int*>(smraw + hg_plan_offset(FP, s.fmax));
-    const unsigned plb = (unsigned)(PLAN_INTS * RG) * 4, frb = (unsigned)(FRN_INTS * s.fmax) * 4;
-    auto copy_plan = [&](int c) {  // thread 0
+        bulk_g2s(As, s.Ah + (size_t)n * FP, fb, bar);
+        bulk_g2s(As + FP, s.Ag + (size_t)n * FP, fb, bar);
+    }
+    __device__ __forceinline__ void copy_plan(int c) const {  // thread 0
+        const unsigned plb = (unsigned)(PLAN_INTS * RG) * 4, frb = (unsigned)(FRN_INTS * s.fmax) * 4;
         fence_proxy_async_all();
         mbar_expect_tx(&bar[1], plb + frb);
         bulk_g2s(Ps, s.plan_hg + (size_t)c * RG * PLAN_INTS, plb, &bar[1]);
         bulk_g2s(Ps + PLAN_INTS * RG, frn_hg_of(s, c), frb, &bar[1]);
-    };
-    const bool fast = FAST;
-    if (t == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        // without level order the first item's plan and planes are copied at once
-        if (fast && (int)blockIdx.x < total) {
-            copy_plan(blockIdx.x);
-            copy_planes(first);
-        }
     }
+};
+template <int N, bool FAST>
+__device__ __forceinline__ void fill_hg_stream_body(const DevState& s, const Geo<N>& G,
+                                                    const HgStage<N>& S, int wr, int total) {
+    __shared__ NbInfo nbis[2];
+    __shared__ int s_next;
+    const int q = Q_FILLHG;
+    const int t = threadIdx.x, RG = S.RG;
+    unsigned long long* bar = S.bar;
+    double *As = S.As, *Fs = S.Fs;
+    int* Ps = S.Ps;
     unsigned phase = 0;  // bit b: parity of bar[b]'s next completion
 
-    if (fast) {
+    if (FAST) {
         __shared__ int srec[2][REC_WORDS];  // records of the current and the next item
         int c = blockIdx.x, rb = 0;
         if (c < total) item_rec_stage(s, c, q, srec[0]);
@@ -1161,32 +1275,41 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, int wr, i
                 if ((bits >> b) & 1u) mbar_wait(&bar[b], (phase >> b) & 1u);
             cp_async_wait_all();
         };
+        if (c >= total) drain(3u);
         while (c < total) {
             const int cn = c + gridDim.x;
             const ItemRec r = item_rec_of(srec[rb]);
-            if (t == 0 && c != (int)blockIdx.x) copy_planes(r.n);
+            if (t == 0 && c != (int)blockIdx.x) S.copy_planes(r.n);
             if (cn < total) item_rec_stage_async(s, cn, q, srec[rb ^ 1]);  // for the next iteration
+            const int nj = r.dx == 1 ? 3 : 6;  // Perfect_Shift_AMR
             if (__syncthreads_or(mbar_wait(&bar[1], (phase >> 1) & 1u) ? 0 : 1)) {
                 if (t == 0) set_error(s, 8 /*AMRLBM_ERR_TIMEOUT*/, 100 + q);
                 drain(3u);
                 break;
             }
             phase ^= 2u;
-            foreign_hg<N>(s, G, Ps + PLAN_INTS * RG, r.nf, true, Fs);  // while the planes land
-            if (__syncthreads_or(mbar_wait(&bar[0], phase & 1u) ? 0 : 1)) {
+            auto landed = [&]() { return !__syncthreads_or(mbar_wait(&bar[0], phase & 1u) ? 0 : 1); };
+            bool ok;
+            if (wr) {  // the whole ring, also to memory
+                foreign_hg<N>(s, G, Ps + PLAN_INTS * RG, r.nf, true, Fs);
+                ok = landed();
+                if (ok) fast_ring_hg<N>(s, G, Ps, r, Fs, As);
+            } else {
+                foreign_stream<N>(s, G, Ps + PLAN_INTS * RG, r.nf, nj, Fs);
+                ok = stream_ring<N>(s, G, Ps, r, nj, Fs, As, landed);
+            }
+            if (!ok) {
                 if (t == 0) set_error(s, 8 /*AMRLBM_ERR_TIMEOUT*/, 100 + q);
                 drain(1u);
                 break;
             }
             phase ^= 1u;
-            // the ring, then Bounce_Back_3/4, on the staged planes (and in memory if wr)
-            fast_ring_hg<N>(s, G, Ps, r, Fs, As, wr != 0);
-            if (t == 0 && cn < total) copy_plan(cn);  // the ring is filled: for the next iteration
             if (r.w3 || r.w4) {
                 bounce_back_staged<N>(s, G, r.n, r.w3, r.w4, As, wr != 0);
                 __syncthreads();
             }
-            stream_block<N>(s, G, r.n, As);
+            if (t == 0 && cn < total) S.copy_plan(cn);  // the ring is filled: for the next iteration
+            stream_block<N>(s, G, r.n, As, StreamCoef(r.dx));
             cp_async_wait_all();  // the next item's record
             __syncthreads();
             c = cn;
@@ -1196,6 +1319,10 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, int wr, i
     }
 
     __syncthreads();  // the mbarriers are initialised
+    // the copies issued at entry land before anything else uses the stage
+    const bool landed = mbar_wait(&bar[0], 0) && mbar_wait(&bar[1], 0);
+    if (!landed && t == 0) set_error(s, 8 /*AMRLBM_ERR_TIMEOUT*/, 100 + q);
+    phase = 3u;
     const int lmin = s.cnt->level_min;
     fill_phase(
         s, q, nbis, &s_next,
@@ -1209,7 +1336,7 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, int wr, i
                 fill_ring_hg<N>(s, G, k, n, 0, Fs);
             }
         },
-        [&](int n, const NbInfo& nbi) { bounce_back<N>(s, G, n, nbi); });
+        [&](int n, const NbInfo& nbi) { bounce_back<N>(s, G, n, nbi.id[3] < 0, nbi.id[4] < 0); });
     const int* flags = fill_flags(s, q);
     if (t == 0) s_next = (int)atomicAdd(&s.queue[4 * q + 1], 1u);
     __syncthreads();
@@ -1219,7 +1346,7 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, int wr, i
         if (t == 0) {
             const unsigned cn = atomicAdd(&s.queue[4 * q + 1], 1u);
             if (!spin_flag(flags + n, s.spin_limit)) set_error(s, 8 /*AMRLBM_ERR_TIMEOUT*/, 200 + q);
-            copy_planes(n);
+            S.copy_planes(n);
             s_next = (int)cn;
         }
         if (__syncthreads_or(mbar_wait(bar, phase & 1u) ? 0 : 1)) {
@@ -1228,24 +1355,35 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, int wr, i
             break;
         }
         phase ^= 1u;
-        stream_block<N>(s, G, n, As);
+        stream_block<N>(s, G, n, As, StreamCoef(__ldg(s.dx + n)));
         c = s_next;
         __syncthreads();
     }
     queue_done(s, q);
 }
-// the unordered and the level-ordered path as two instantiations, as
-// k_fill_c. The item count and the first item's block are loaded with the
-// level-order flags, so that the first bulk copies wait for one round trip
-// only (first: block of item blockIdx.x without level order)
+// The unordered and the level-ordered path as two instantiations, as
+// k_fill_c. A CTA's first item is item blockIdx.x of the work order unless
+// the fill needs level order, so its plan, then its planes, are copied at
+// entry, before the flags that tell which path runs arrive (the pools hold
+// max_blks + 1 blocks and plans: any index the work order holds is in range).
 template <int N>
-__global__ void __launch_bounds__(256, 3) k_fill_hg_stream(DevState s, int wr) {
+__global__ void __launch_bounds__(256, 3)
+    k_fill_hg_stream(const __grid_constant__ DevState s, int wr) {
+    extern __shared__ __align__(128) unsigned char smraw[];
+    const Geo<N> G(s);
+    const HgStage<N> S(s, G, smraw);
     const int total = s.lvl_off[AMR_MAXLV];
-    const int first = (int)blockIdx.x <= s.max_blks ? __ldg(s.lvl_leaf + blockIdx.x) : 0;
+    if (threadIdx.x == 0) {
+        mbar_init(&S.bar[0], 1);
+        mbar_init(&S.bar[1], 1);
+        const int c = min((int)blockIdx.x, s.max_blks);
+        S.copy_plan(c);
+        S.copy_planes(__ldg(s.lvl_leaf + c));
+    }
     if (fast_fill(s, Q_FILLHG))
-        fill_hg_stream_body<N, true>(s, wr, total, first);
+        fill_hg_stream_body<N, true>(s, G, S, wr, total);
     else
-        fill_hg_stream_body<N, false>(s, wr, total, first);
+        fill_hg_stream_body<N, false>(s, G, S, wr, total);
 }
 
 
@@ -1269,7 +1407,7 @@ __global__ void __launch_bounds__(256, 2) k_collide(DevState s) {
     for (int m = blockIdx.x; m < nleaf; m += gridDim.x) {
         const int n = s.leaf[m];
         load_tile_c<N>(s, G, n, T);
-        collide_block<N, false, false, false, BGK, BATCH>(s, G, n, T, s.Bh + (size_t)n * 9 * G.bplane,
+        collide_block<N, false, false, false, BGK, BATCH>(s, G, n, __ldg(s.dx + n), T, s.Bh + (size_t)n * 9 * G.bplane,
                                                    s.Bg + (size_t)n * 9 * G.bplane);
         __syncthreads();
     }
@@ -1284,7 +1422,7 @@ __global__ void __launch_bounds__(256, 2) k_macro_g(DevState s) {
     for (int m = blockIdx.x; m < nleaf; m += gridDim.x) {
         const int n = s.leaf[m];
         load_tile_c<N>(s, G, n, T);
-        err_reduce(s, n, macro_g_block<N, false, BATCH>(s, G, n, T, s.Bg + (size_t)n * 9 * G.bplane), red);
+        err_reduce(s, n, macro_g_block<N, false, BATCH>(s, G, n, __ldg(s.dx + n), T, s.Bg + (size_t)n * 9 * G.bplane), red);
         __syncthreads();
     }
 }
@@ -1454,7 +1592,10 @@ void launch_fill_c(const DevState& s, const LaunchCfg& lc, cudaStream_t st, int 
 }
 
 void launch_fill_hg_stream(const DevState& s, const LaunchCfg& lc, cudaStream_t st, int write_ring) {
-    const int nt = block_threads(s);
+    // at least 128 threads: the ring's gathers, several values per cell of a
+    // small block, outnumber its cells (8x8 blocks, 189 leaves: 14.4 us per
+    // launch against 19.8 us with 64)
+    const int nt = block_threads(s) < 128 ? 128 : block_threads(s);
     // mbarriers, h and g planes, foreign values, the staged plan
     const size_t sm = hg_plan_offset(9 * (size_t)s.aplane, s.fmax) +
                       sizeof(int) * (size_t)plan_stage_ints(ring1_len(s.nx, s.ny), s.fmax);
