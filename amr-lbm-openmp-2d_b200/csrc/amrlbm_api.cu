@@ -563,9 +563,7 @@ int amrlbm_create(const amrlbm_params* p, amrlbm_ctx** out) {
     AL(plan_c2, int, NB * PLAN_INTS * (size_t)(4 * (nx + ny) + 16));
     AL(plan_c1, int, NB * PLAN_INTS * (size_t)(2 * (nx + ny) + 4));
     AL(plan_hg, int, NB * PLAN_INTS * (size_t)(2 * (nx + ny) + 4));
-    // a fine leaf reads at most half a side plus two cells of a coarser
-    // neighbour's ring per side, and five cells per corner
-    s.fmax = 2 * (nx > ny ? nx : ny) + 28;
+    s.fmax = foreign_slots(nx, ny);
     AL(frn_c, int, NB * 11 * (size_t)s.fmax);
     AL(frn_hg, int, NB * 11 * (size_t)s.fmax);
     AL(fillinfo, int, NQUEUES);

@@ -47,6 +47,7 @@ void launch_regrid_topo(const DevState& s, cudaStream_t st, int mode, int lmin, 
                         int set_levels);
 // neighbour records and ghost-cell fill plans of the leaves in work order;
 // after every change of the topology
+int foreign_slots(int nx, int ny);  // foreign cells per leaf, at most (DevState::fmax)
 void launch_build_plans(const DevState& s, const LaunchCfg& lc, cudaStream_t st);
 void launch_prolong(const DevState& s, const LaunchCfg& lc, cudaStream_t st);
 void launch_zero_children(const DevState& s, const LaunchCfg& lc, cudaStream_t st);

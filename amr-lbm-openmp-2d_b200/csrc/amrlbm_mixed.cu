@@ -17,8 +17,7 @@
 // over the items in work order. Items do not wait for one another where the
 // plans' foreign cells make every ring depend on interiors only; where a
 // coarse-to-fine stencil reads a coarser neighbour's ring cell that is itself
-// coarse-to-fine or a wall cell, the launch takes the items in level order
-// (see claim).
+// coarse-to-fine, the launch takes the items in level order (see claim).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -155,6 +154,20 @@ __device__ __forceinline__ void dec_a9(const MpState& m, const Geo<N>& G, int f,
 #pragma unroll
     for (int q = 2; q <= 9; ++q) v[q - 1] = dec<FMT>(__ldg(D + (unsigned)(q - 1) * G.aplane)) * is + rq(q) * rest;
 }
+// the eight deviation words of a cell of A (offset off of its first plane)
+// from its populations v
+template <int FMT>
+__device__ __forceinline__ void enc_words(const MpState& m, int f, unsigned off, int aplane,
+                                          const float* v, unsigned short* w) {
+    const float sc = f ? m.sg : m.sh;
+    float e = 0.f;  // h: rounding error carried (mass_encode)
+#pragma unroll
+    for (int q = 2; q <= 9; ++q) {
+        const float x = (v[q - 1] - rq(q) * v[0]) * sc - e;
+        w[q - 2] = enc_sr<FMT>(x, (off + (unsigned)((q - 1) * aplane)) * 2u + f);
+        if (f == 0) e = dec<FMT>(w[q - 2]) - x;
+    }
+}
 // writes the 9 populations v of field f of cell (x, y) of block n into A;
 // rest (if given): v[0] before its rounding to FP32
 template <int N, int FMT>
@@ -164,15 +177,10 @@ __device__ __forceinline__ void enc_a9(const MpState& m, const Geo<N>& G, int f,
     if (rest) v[0] = f32_sr(*rest, (unsigned)off * 2u + f + 0x51ed27u);
     (f ? m.A1g : m.A1h)[off - (size_t)8 * G.aplane * n] = v[0];
     unsigned short* D = (f ? m.Adg : m.Adh) + off;
-    const float sc = f ? m.sg : m.sh;
-    float e = 0.f;  // h: rounding error carried (mass_encode)
+    unsigned short w[8];
+    enc_words<FMT>(m, f, (unsigned)off, G.aplane, v, w);
 #pragma unroll
-    for (int q = 2; q <= 9; ++q) {
-        const float x = (v[q - 1] - rq(q) * v[0]) * sc - e;
-        const unsigned short w = enc_sr<FMT>(x, (unsigned)(off + (size_t)(q - 1) * G.aplane) * 2u + f);
-        D[(size_t)(q - 1) * G.aplane] = w;
-        if (f == 0) e = dec<FMT>(w) - x;
-    }
+    for (int q = 2; q <= 9; ++q) D[(size_t)(q - 1) * G.aplane] = w[q - 2];
 }
 
 // Biquadratic_from_Fine / _Coarse (Interpolations.f90:2-138) of a plan entry
@@ -200,6 +208,19 @@ __device__ __forceinline__ float foreign_cf(const int* fb, int fmax, int j, cons
 #pragma unroll
     for (int i = 0; i < 9; ++i) g[i] = __ldg(C + (unsigned)fb[(1 + i) * fmax + j]);
     return combine_f(meta, g);
+}
+// the item's foreign cells into Fs, those behind a wall (of the value before
+// it) after the others. Ends with a barrier.
+__device__ __forceinline__ void foreign_all_cf(const int* fb, int fmax, const ItemRec& r,
+                                               const float* C, float* Fs) {
+    for (int j = threadIdx.x; j < r.nd; j += blockDim.x) Fs[j] = foreign_cf(fb, fmax, j, C);
+    __syncthreads();
+    if (r.nf == r.nd) return;
+    for (int j = r.nd + threadIdx.x; j < r.nf; j += blockDim.x) {
+        const unsigned w = (unsigned)fb[fmax + j];
+        Fs[j] = (w & kIndirect) ? Fs[w & ~kIndirect] : __ldg(C + w);
+    }
+    __syncthreads();
 }
 
 // the C ring of width w of item k (block n) on the tile T (pool layout of
@@ -456,7 +477,7 @@ __device__ __forceinline__ void enc_b9(const MpState& m, const Geo<N>& G, int f,
 template <int N>
 struct K1Stage {
     static constexpr int R = 4 * (N + N) + 16;  // ring2_len
-    static constexpr int FMAX = 2 * N + 28;     // foreign slots per leaf
+    static constexpr int FMAX = foreign_max(N, N);  // foreign slots per leaf
     static constexpr int TILE = cplane_of(N) * 4, DEV = 9 * N * N * 2, REST = N * N * 4;
     static constexpr int PLAN = R * PLAN_INTS * 4, FRN = FMAX * FRN_INTS * 4;
     static constexpr int BYTES = TILE + 2 * DEV + 2 * REST + PLAN + FRN;
@@ -515,8 +536,7 @@ __global__ void __launch_bounds__(N * N, (N == 16 ? 3 : 8)) k_mp_collide(const _
             const int n = r.n;
             load_tile<N>(s, G, n, T);
             const int* fb = s.frn_c + (size_t)k * s.fmax * FRN_INTS;
-            for (int j = t; j < r.nf; j += blockDim.x) Fs[j] = foreign_cf(fb, s.fmax, j, m.C);
-            __syncthreads();
+            foreign_all_cf(fb, s.fmax, r, m.C, Fs);
             wait_for_coarser(s, Q_FILLC, k);
             ring_c<N>(s, G, s.plan_c2 + (size_t)k * R * PLAN_INTS, R, 2, r, Fs, T, true);
             walls_c<N>(s, G, n, 2, r.w3, r.w4, T);
@@ -569,8 +589,7 @@ __global__ void __launch_bounds__(N * N, (N == 16 ? 3 : 8)) k_mp_collide(const _
         const ItemRec r = item_rec_of(rec[st]);
         const int n = r.n;
         const int* fb = reinterpret_cast<const int*>(S + SL::O_FR);
-        for (int j = t; j < r.nf; j += blockDim.x) Fs[j] = foreign_cf(fb, s.fmax, j, m.C);
-        __syncthreads();
+        foreign_all_cf(fb, s.fmax, r, m.C, Fs);
         ring_c<N>(s, G, reinterpret_cast<const int*>(S + SL::O_PL), R, 2, r, Fs, T, false);
         walls_c<N>(s, G, n, 2, r.w3, r.w4, T);
         // the next item's copies, now that its record is in
@@ -608,7 +627,7 @@ __global__ void __launch_bounds__(N * N, (N == 16 ? 3 : 8)) k_mp_collide(const _
 // 8-byte cp.async (a block's 9 planes start on 8-byte boundaries only).
 template <int N>
 struct K2Stage {
-    static constexpr int AP = (N + 2) * (N + 2), R = 2 * (N + N) + 4, FMAX = 2 * N + 28;
+    static constexpr int AP = (N + 2) * (N + 2), R = 2 * (N + N) + 4, FMAX = foreign_max(N, N);
     static constexpr int DEV = 9 * AP * 2, REST = AP * 4, PLAN = R * PLAN_INTS * 4,
                          FRN = FMAX * FRN_INTS * 4;
     static constexpr int O_DG = DEV, O_RH = 2 * DEV, O_RG = O_RH + REST, O_PL = O_RG + REST,
@@ -638,8 +657,8 @@ __device__ void hg_item(const DevState& s, const Geo<N>& G, int k, const ItemRec
     const int t = threadIdx.x, n = r.n, RG = ring1_len(N, N), fmax = s.fmax;
     const MpState& m = s.mp;
     // foreign cells: one thread per (slot, field and population)
-    for (int idx = t; idx < 18 * r.nf; idx += blockDim.x) {
-        const int j = idx % r.nf, fq = idx / r.nf, f = fq / 9, q = fq % 9 + 1;
+    for (int idx = t; idx < 18 * r.nd; idx += blockDim.x) {
+        const int j = idx % r.nd, fq = idx / r.nd, f = fq / 9, q = fq % 9 + 1;
         const int meta = fb[j];
         float v;
         if (plan_kind(meta) == 1) {
@@ -653,6 +672,33 @@ __device__ void hg_item(const DevState& s, const Geo<N>& G, int k, const ItemRec
         Fs[fq * fmax + j] = v;
     }
     __syncthreads();
+    // those behind a wall (Bounce_Back_3/4, BC_Cell.f90:2-42), rounded as the
+    // neighbour's ring in memory is: one thread per (slot, field)
+    const int n1 = r.nf - r.nd;
+    if (n1) {
+        for (int idx = t; idx < 2 * n1; idx += blockDim.x) {
+            const int j = r.nd + idx % n1, f = idx / n1;
+#pragma unroll 1
+            for (int q = 1; q <= 9; ++q) {
+                const int J = q > 1 ? (q - 2) + 4 * ((q / 2) % 2) : 1;
+                const int col = 1 + ((fb[j] & 8) ? -1 : 1) * d_ex(q) * d_ey(q);
+                const unsigned wd = (unsigned)fb[(1 + col) * fmax + j];
+                Fs[(f * 9 + q - 1) * fmax + j] = (wd & kIndirect)
+                                                     ? Fs[(f * 9 + J - 1) * fmax + (wd & ~kIndirect)]
+                                                     : dec_a<N, FMT>(m, G, f, wd, J);
+            }
+            float v[9];
+#pragma unroll
+            for (int q = 0; q < 9; ++q) v[q] = Fs[(f * 9 + q) * fmax + j];
+            unsigned short w[8];
+            enc_words<FMT>(m, f, (unsigned)fb[10 * fmax + j], G.aplane, v, w);
+            Fs[f * 9 * fmax + j] = v[0];
+#pragma unroll
+            for (int q = 2; q <= 9; ++q)
+                Fs[(f * 9 + q - 1) * fmax + j] = dec<FMT>(w[q - 2]) * (f ? m.isg : m.ish) + rq(q) * v[0];
+        }
+        __syncthreads();
+    }
     if (!fast) wait_for_coarser(s, Q_FILLHG, k);
     // the ring: copies per (cell, field), interpolated cells per (cell, population),
     // populations fastest, so that a cell's 9 threads share each source's rest load
@@ -898,8 +944,7 @@ __global__ void __launch_bounds__(N * N) k_mp_tail(const __grid_constant__ DevSt
         const int n = r.n;
         load_tile<N>(s, G, n, T);
         const int* fb = s.frn_c + (size_t)k * s.fmax * FRN_INTS;
-        for (int j = t; j < r.nf; j += blockDim.x) Fs[j] = foreign_cf(fb, s.fmax, j, m.C);
-        __syncthreads();
+        foreign_all_cf(fb, s.fmax, r, m.C, Fs);
         if (!fast) wait_for_coarser(s, Q_FILLC1, k);
         // through L2 also without level order: measured faster here (the ring
         // of one width has little reuse of its sources)

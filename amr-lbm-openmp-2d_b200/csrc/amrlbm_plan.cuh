@@ -18,6 +18,23 @@ __device__ __forceinline__ int ghost_dir(int x, int y, int nx, int ny) {
     return yb ? 3 : 4;
 }
 
+// Which populations of a ghost cell in direction d streaming reads: of the
+// cells beside it, those that move from it into the block (digits 0-2) and,
+// for Lax-Wendroff only, the opposite ones (digits 3-5); 0: none. Three
+// (six) of the nine on a side, one (two) in a corner.
+__device__ __forceinline__ unsigned stream_pops(int d) {
+    switch (d) {
+        case 1: return 0x874962u;
+        case 2: return 0x962874u;
+        case 3: return 0x985763u;
+        case 4: return 0x763985u;
+        case 5: return 0x008006u;
+        case 6: return 0x007009u;
+        case 7: return 0x009007u;
+        default: return 0x006008u;
+    }
+}
+
 // per-direction neighbour data of the block being filled, loaded once into
 // shared memory: resolved id, its level, leaf flag and first child (index 0:
 // the block itself); per fill q: wait[q], the directions whose rings a
@@ -27,6 +44,7 @@ struct NbInfo {
     int bi, bj, dx;
     int wait[NQUEUES];
     int nf[NQUEUES];
+    int nd;  // foreign cells that are not behind a wall
     // plan entries stored first: na of kinds 1 and -1, then n2 of kind 2, then
     // n3 of kind 3 (then those without a plan)
     int na[NQUEUES], n2[NQUEUES], n3[NQUEUES];
@@ -208,8 +226,22 @@ __host__ __device__ __forceinline__ int ring1_len(int nx, int ny) { return 2 * (
 // neighbour's ghost cell that is a copy or a fine-to-coarse value of
 // interiors, which the item evaluates itself before its coarse-to-fine
 // cells. A foreign record (FRN_INTS ints, plane by plane over fmax slots)
-// holds that ghost cell's plan (meta word, 9 sources) and its offset.
+// holds that ghost cell's plan (meta word, 9 sources) and its offset; the
+// meta word's bits 8- hold the direction (1..8) of the neighbour whose ghost
+// cell it is. Slots 0..nd-1 read interiors only. Slots nd..nf-1 are the
+// neighbour's cells behind a wall, whose values are those of the row before
+// the wall, interior cells or slots below nd: of C the value of the same
+// column (kind 1), of h and g (kind kWall, bit 3: the top wall) population by
+// population the opposite one of a column beside it (Bounce_Back_3/4; sources
+// 0-2: the columns x-1, x, x+1).
 constexpr unsigned kIndirect = 0x80000000u;
+constexpr int kWall = 4;
+// foreign cells of a leaf: at most half a side plus four cells of a coarser
+// neighbour's ring on each of the two sides its siblings leave, five cells
+// at each of three corners
+__host__ __device__ constexpr int foreign_max(int nx, int ny) {
+    return 2 * (nx > ny ? nx : ny) + 28;
+}
 constexpr int FRN_INTS = 11;
 
 __device__ __forceinline__ int ring1_index(int x, int y, int nx, int ny) {
@@ -224,17 +256,18 @@ constexpr int REC_NA = (int)(offsetof(NbInfo, na) / sizeof(int));
 constexpr int REC_N2 = (int)(offsetof(NbInfo, n2) / sizeof(int));
 constexpr int REC_N3 = (int)(offsetof(NbInfo, n3) / sizeof(int));
 constexpr int REC_DX = (int)(offsetof(NbInfo, dx) / sizeof(int));
+constexpr int REC_ND = (int)(offsetof(NbInfo, nd) / sizeof(int));
 
 // what an item of fill q needs from its record: block, foreign cells, plan
 // entry classes, walls (id[3], id[4] < 0), cell size; staged in shared memory
-// by threads 0..7 (REC_WORDS words), read from there by every thread
+// by threads 0..8 (REC_WORDS words), read from there by every thread
 struct ItemRec {
     int n, nf, na, n2, n3;
     bool w3, w4;
-    int dx;
+    int dx, nd;
 };
-constexpr int REC_WORDS = 8;
-// word t of an item record: n, nf, na, n2, n3, id[3] (bottom), id[4] (top), dx
+constexpr int REC_WORDS = 9;
+// word t of an item record: n, nf, na, n2, n3, id[3] (bottom), id[4] (top), dx, nd
 __device__ __forceinline__ const int* item_rec_word(const DevState& s, int c, int q, int t) {
     const int off = t == 0   ? 0
                     : t == 1 ? REC_NF + q
@@ -242,6 +275,7 @@ __device__ __forceinline__ const int* item_rec_word(const DevState& s, int c, in
                     : t == 3 ? REC_N2 + q
                     : t == 4 ? REC_N3 + q
                     : t == 7 ? REC_DX
+                    : t == 8 ? REC_ND
                              : t - 2;
     return s.nbinfo + (size_t)c * NBI_STRIDE + off;
 }
@@ -249,7 +283,7 @@ __device__ __forceinline__ void item_rec_stage(const DevState& s, int c, int q, 
     const int t = threadIdx.x;
     if (t < REC_WORDS) dst[t] = __ldg(item_rec_word(s, c, q, t));
 }
-// the same without waiting for the loads: threads 0..7 gather the words with
+// the same without waiting for the loads: threads 0..8 gather the words with
 // cp.async and call cp_async_wait_all before the barrier that precedes the
 // first read of dst (thread 0, which copies word 0, may read it after its
 // own wait)
@@ -267,6 +301,7 @@ __device__ __forceinline__ ItemRec item_rec_of(const int* w) {
     o.w3 = w[5] < 0;
     o.w4 = w[6] < 0;
     o.dx = w[7];
+    o.nd = w[8];
     return o;
 }
 

@@ -42,10 +42,13 @@ namespace {
 // reference fills one level earlier. Where such a ring cell is a copy or a
 // fine-to-coarse value, it becomes a foreign cell of the reading leaf: the
 // leaf evaluates it from its plan, with the operations the neighbour's own
-// fill uses, so the two leaves need not be ordered. Where it is itself
-// coarse-to-fine or a wall cell, or a fill meets a level jump, the fill is
-// marked as needing level order (fillinfo[q]), and the record's wait mask
-// names the neighbours whose rings the leaf waits for then.
+// fill uses, so the two leaves need not be ordered. A coarser neighbour's
+// cell behind a wall is a foreign cell too, evaluated after those from the
+// row before the wall (a bubble refined down to a wall: one such problem of a
+// batch had all of it filled in level order, 1,495 us per step of 17,568
+// leaves against 817). Where it is itself coarse-to-fine, or a fill meets a
+// level jump, the fill is marked as needing level order (fillinfo[q]), and
+// the record's wait mask names the neighbours whose rings the leaf waits for.
 __device__ void load_nbinfo(const DevState& s, int n, NbInfo& r) {
     for (int j = 0; j < 8; ++j) {
         const int b = s.nbr[8 * n + j];
@@ -62,6 +65,7 @@ __device__ void load_nbinfo(const DevState& s, int n, NbInfo& r) {
     r.bj = s.bj[n];
     r.dx = s.dx[n];
     for (int q = 0; q < NQUEUES; ++q) r.wait[q] = r.nf[q] = 0;
+    r.nd = 0;
 }
 
 // One pass over the ghost cells of rings 1-2 serves all three fills: a cell's
@@ -73,7 +77,7 @@ __global__ void __launch_bounds__(128, 8) k_build_plans(DevState s) {
     extern __shared__ int tab[];  // [9][ring1_len]: foreign cell -> slot
     __shared__ NbInfo nbi;
     __shared__ NbInfo cnb[9];     // coarser neighbours' records
-    __shared__ int nfs;
+    __shared__ int nfs, nds;
     __shared__ int cls_n[2][4], cls_f[2][4];  // [C2 | ring-1 plans][class]: count, fill
     if (!s.cnt->topo_changed) return;  // the mesh did not change: the plans stand
     const int nx = G.nx, ny = G.ny, R2 = ring2_len(nx, ny), R1 = ring1_len(nx, ny);
@@ -97,13 +101,19 @@ __global__ void __launch_bounds__(128, 8) k_build_plans(DevState s) {
         auto offc = [&](int blk, int xx, int yy) -> long long { return (long long)G.c(blk, xx, yy); };
         // ghost cell (xx,yy) of block blk, read from direction d: 1 a foreign
         // cell (the coarser neighbour's neighbour on that side has its level:
-        // a copy or a fine-to-coarse value), -1 a coarser ring cell that is
-        // not, 0 not a coarser neighbour's ghost cell
+        // a copy or a fine-to-coarse value), 2 one behind a wall (the
+        // neighbour's ghost cells beside it, if it reads any, are of the first
+        // kind), -1 any other coarser ring cell, 0 not a coarser neighbour's
+        // ghost cell
         auto foreign = [&](int d, int blk, int xx, int yy) {
             const bool ring = xx < 1 || xx > nx || yy < 1 || yy > ny;
             if (!ring || blk != nbi.id[d] || nbi.lev[d] != L - 1) return 0;
-            const int dd = ghost_dir(xx, yy, nx, ny);
-            return (nbi.leaf[d] && cnb[d].id[dd] > 0 && cnb[d].lev[dd] == L - 1) ? 1 : -1;
+            const NbInfo& c = cnb[d];
+            auto level = [&](int dd) { return c.id[dd] > 0 && c.lev[dd] == L - 1; };
+            if (!nbi.leaf[d]) return -1;
+            if ((yy < 1 && c.id[3] < 0) || (yy > ny && c.id[4] < 0))
+                return ((xx > 1 || level(1)) && (xx < nx || level(2))) ? 2 : -1;
+            return level(ghost_dir(xx, yy, nx, ny)) ? 1 : -1;
         };
         // 1: mark the foreign cells; anything else makes the fills wait
         for (int i = t; i < R2; i += blockDim.x) {
@@ -115,7 +125,12 @@ __global__ void __launch_bounds__(128, 8) k_build_plans(DevState s) {
             ghost_plan(nbi, nx, ny, L, d, x, y,
                        [&](int blk, int xx, int yy) -> long long {
                            const int f = foreign(d, blk, xx, yy);
-                           if (f > 0) tab[d * R1 + ring1_index(xx, yy, nx, ny)] = -2;
+                           if (f > 0) tab[d * R1 + ring1_index(xx, yy, nx, ny)] = -1 - f;
+                           if (f == 2) {  // and the ghost cells beside it
+                               const int yi = yy < 1 ? 1 : ny;
+                               if (xx <= 1) tab[d * R1 + ring1_index(0, yi, nx, ny)] = -2;
+                               if (xx >= nx) tab[d * R1 + ring1_index(nx + 1, yi, nx, ny)] = -2;
+                           }
                            if (f < 0) {
                                atomicOr(&nbi.wait[Q_FILLC], 1 << d);
                                if (r1) {
@@ -143,14 +158,17 @@ __global__ void __launch_bounds__(128, 8) k_build_plans(DevState s) {
         // 2: number the marked cells and write their records (C and A offsets)
         int* fc = s.frn_c + (size_t)k * fmax * FRN_INTS;
         int* fa = s.frn_hg + (size_t)k * fmax * FRN_INTS;
+        auto next_slot = [&]() {
+            const int j = atomicAdd(&nfs, 1);
+            if (j < fmax) return j;
+            set_error(s, 7 /*AMRLBM_ERR_STATE*/, n);  // not reached: fmax bounds the cells a leaf reads
+            return -1;
+        };
         for (int i = t; i < 9 * R1; i += blockDim.x) {
             if (tab[i] != -2) continue;
-            const int j = atomicAdd(&nfs, 1);
+            const int j = next_slot();
             tab[i] = j;
-            if (j >= fmax) {  // not reached: fmax bounds the cells a leaf reads
-                set_error(s, 7 /*AMRLBM_ERR_STATE*/, n);
-                continue;
-            }
+            if (j < 0) continue;
             const int d = i / R1;
             int xx, yy;
             ring1_xy(i % R1, nx, ny, xx, yy);
@@ -170,12 +188,40 @@ __global__ void __launch_bounds__(128, 8) k_build_plans(DevState s) {
             fa[10 * fmax + j] = (int)G.a(nbi.id[d], 1, xx, yy);
         }
         __syncthreads();
+        if (t == 0) nds = nfs;
+        __syncthreads();
+        // those behind a wall: the columns x-1, x, x+1 (within the ring) of the
+        // row before it
+        for (int i = t; i < 9 * R1; i += blockDim.x) {
+            if (tab[i] != -3) continue;
+            const int j = next_slot();
+            tab[i] = j;
+            if (j < 0) continue;
+            const int d = i / R1, blk = nbi.id[d];
+            int xx, yy;
+            ring1_xy(i % R1, nx, ny, xx, yy);
+            const int yi = yy < 1 ? 1 : ny;
+            for (int m = 0; m < 10; ++m) fc[m * fmax + j] = fa[m * fmax + j] = 0;
+            fc[j] = 2 | (d << 8);  // kind 1
+            fa[j] = (kWall + 1) | (yy < 1 ? 0 : 8) | (d << 8);
+            for (int m = 0; m < 3; ++m) {
+                const int x2 = min(max(xx - 1 + m, 0), nx + 1);
+                const bool in = x2 >= 1 && x2 <= nx;
+                const int w = (int)(kIndirect | (unsigned)tab[d * R1 + ring1_index(x2, yi, nx, ny)]);
+                fa[(1 + m) * fmax + j] = in ? (int)G.a(blk, 1, x2, yi) : w;
+                if (m == 1) fc[fmax + j] = in ? (int)offc(blk, x2, yi) : w;
+            }
+            fc[10 * fmax + j] = (int)offc(blk, xx, yy);
+            fa[10 * fmax + j] = (int)G.a(blk, 1, xx, yy);
+        }
+        __syncthreads();
         if (t < NQUEUES) {
             nbi.nf[t] = nfs;
             const int pt = (t == Q_FILLC) ? 0 : 1;
             nbi.na[t] = cls_n[pt][0];
             nbi.n2[t] = cls_n[pt][1];
             nbi.n3[t] = cls_n[pt][2];
+            if (t == 0) nbi.nd = nds;
             if (nbi.wait[t]) atomicOr(&s.fillinfo[t], 1);
         }
         // 3: the plans, foreign cells by slot
@@ -341,23 +387,65 @@ __device__ __forceinline__ const int* frn_c_of(const DevState& s, int k) {
 __device__ __forceinline__ const int* frn_hg_of(const DevState& s, int k) {
     return s.frn_hg + (size_t)k * s.fmax * FRN_INTS;
 }
-// foreign cells of a C fill (records fb, in memory or shared memory) into
-// Fs; ends with a barrier when there are any (nf is block-uniform)
+// a foreign cell behind a wall (slots nd..nf-1) of C, or population q of one
+// of h or g (plane stride AP; F: the field's values of the slots below nd,
+// planes of fmax)
+__device__ __forceinline__ double foreign_wall_c(const int* fb, int fmax, int j, const double* C,
+                                                 const double* F, bool live) {
+    const unsigned w = (unsigned)fb[(live ? 1 : 10) * fmax + j];
+    if (!live) return ldcg(C + w);
+    return (w & kIndirect) ? F[w & ~kIndirect] : __ldg(C + w);
+}
+// the column (0-2) and the population that a wall cell's population q takes
+__device__ __forceinline__ int wall_source(int meta, int q, int& J) {
+    J = q > 1 ? (q - 2) + 4 * ((q / 2) % 2) : 1;
+    return 1 + ((meta & 8) ? -1 : 1) * d_ex(q) * d_ey(q);
+}
+__device__ __forceinline__ double foreign_wall_hg(const int* fb, int fmax, int j, const double* A, int AP,
+                                                  int q, const double* F, bool live) {
+    if (!live) return ldcg(A + (unsigned)fb[10 * fmax + j] + (size_t)(q - 1) * AP);
+    int J;
+    const unsigned w = (unsigned)fb[(1 + wall_source(fb[j], q, J)) * fmax + j];
+    return (w & kIndirect) ? F[(J - 1) * fmax + (int)(w & ~kIndirect)]
+                           : __ldg(A + w + (size_t)(J - 1) * AP);
+}
+// the item's foreign cells (nf, the first nd of them not behind a wall); live:
+// the coarser neighbours' rings are filled in this launch
+struct Foreign {
+    const int* fb;
+    int nf, nd;
+    bool live;
+};
+// foreign cells of a C fill (records in memory or shared memory) into Fs;
+// ends with a barrier when there are any (nf is block-uniform)
 template <int N>
-__device__ void foreign_c(const DevState& s, const int* fb, int nf, bool live, double* Fs) {
-    if (nf == 0) return;
-    for (int j = threadIdx.x; j < nf; j += blockDim.x) Fs[j] = foreign_value(fb, s.fmax, j, s.C, 0, live);
+__device__ __forceinline__ void foreign_c(const DevState& s, const Foreign& w, double* Fs) {
+    if (w.nf == 0) return;
+    for (int j = threadIdx.x; j < w.nd; j += blockDim.x)
+        Fs[j] = foreign_value(w.fb, s.fmax, j, s.C, 0, w.live);
+    __syncthreads();
+    if (w.nf == w.nd) return;
+    for (int j = w.nd + threadIdx.x; j < w.nf; j += blockDim.x)
+        Fs[j] = foreign_wall_c(w.fb, s.fmax, j, s.C, Fs, w.live);
     __syncthreads();
 }
 // the same for the h/g fill: one thread per (slot, field and population)
 template <int N>
-__device__ void foreign_hg(const DevState& s, const Geo<N>& G, const int* fb, int nf, bool live,
-                           double* Fs) {
-    if (nf == 0) return;
-    for (int idx = threadIdx.x; idx < 18 * nf; idx += blockDim.x) {
-        const int j = idx % nf, fq = idx / nf;
-        Fs[fq * s.fmax + j] = foreign_value(fb, s.fmax, j, (fq >= 9) ? s.Ag : s.Ah,
-                                            (size_t)(fq % 9) * G.aplane, live);
+__device__ __forceinline__ void foreign_hg(const DevState& s, const Geo<N>& G, const Foreign& w,
+                                           double* Fs) {
+    if (w.nf == 0) return;
+    for (int idx = threadIdx.x; idx < 18 * w.nd; idx += blockDim.x) {
+        const int j = idx % w.nd, fq = idx / w.nd;
+        Fs[fq * s.fmax + j] =
+            foreign_value(w.fb, s.fmax, j, (fq >= 9) ? s.Ag : s.Ah, (size_t)(fq % 9) * G.aplane, w.live);
+    }
+    __syncthreads();
+    const int n1 = w.nf - w.nd;
+    if (n1 == 0) return;
+    for (int idx = threadIdx.x; idx < 18 * n1; idx += blockDim.x) {
+        const int j = w.nd + idx % n1, fq = idx / n1, f = fq / 9;
+        Fs[fq * s.fmax + j] = foreign_wall_hg(w.fb, s.fmax, j, f ? s.Ag : s.Ah, G.aplane, fq % 9 + 1,
+                                              Fs + f * 9 * s.fmax, w.live);
     }
     __syncthreads();
 }
@@ -781,37 +869,30 @@ struct StreamCoef {
     }
 };
 
-// Which populations of a ghost cell in direction d streaming reads: of the
-// cells beside it, those that move from it into the block (digits 0-2) and,
-// for Lax-Wendroff only, the opposite ones (digits 3-5); 0: none. Three
-// (six) of the nine on a side, one (two) in a corner.
-__device__ __forceinline__ unsigned stream_pops(int d) {
-    switch (d) {
-        case 1: return 0x874962u;
-        case 2: return 0x962874u;
-        case 3: return 0x985763u;
-        case 4: return 0x763985u;
-        case 5: return 0x008006u;
-        case 6: return 0x007009u;
-        case 7: return 0x009007u;
-        default: return 0x006008u;
-    }
-}
-
-// Foreign cells of an h/g item (records fb) into Fs[field and population]
-// [slot]: the populations that streaming reads (nj digits of stream_pops).
-// Ends with a barrier when there are any (nf is block-uniform).
+// Foreign cells of an h/g item into Fs[field and population][slot]: the
+// populations that streaming reads (nj digits of stream_pops; where some are
+// behind a wall and take the opposite population, both halves). Ends with a
+// barrier when there are any (nf is block-uniform).
 template <int N>
-__device__ __forceinline__ void foreign_stream(const DevState& s, const Geo<N>& G, const int* fb,
-                                               int nf, int nj, double* Fs) {
-    if (nf == 0) return;
-    const int fmax = s.fmax;
-    for (int u = threadIdx.x; u < 2 * nj * nf; u += blockDim.x) {
-        const int j = u % nf, v = u / nf, f = v >= nj, m = f ? v - nj : v;
-        const int q = (int)(stream_pops(fb[j] >> 8) >> (4 * m)) & 15;
+__device__ __forceinline__ void foreign_stream(const DevState& s, const Geo<N>& G, const Foreign& w,
+                                               int nj, double* Fs) {
+    if (w.nf == 0) return;
+    const int fmax = s.fmax, n1 = w.nf - w.nd, nk = n1 ? 6 : nj;
+    for (int u = threadIdx.x; u < 2 * nk * w.nd; u += blockDim.x) {
+        const int j = u % w.nd, v = u / w.nd, f = v >= nk, m = f ? v - nk : v;
+        const int q = (int)(stream_pops(w.fb[j] >> 8) >> (4 * m)) & 15;
         if (q)
             Fs[(f * 9 + q - 1) * fmax + j] =
-                foreign_value(fb, fmax, j, f ? s.Ag : s.Ah, (size_t)(q - 1) * G.aplane, true);
+                foreign_value(w.fb, fmax, j, f ? s.Ag : s.Ah, (size_t)(q - 1) * G.aplane, true);
+    }
+    __syncthreads();
+    if (n1 == 0) return;
+    for (int u = threadIdx.x; u < 2 * nj * n1; u += blockDim.x) {
+        const int j = w.nd + u % n1, v = u / n1, f = v >= nj, m = f ? v - nj : v;
+        const int q = (int)(stream_pops(w.fb[j] >> 8) >> (4 * m)) & 15;
+        if (q)
+            Fs[(f * 9 + q - 1) * fmax + j] = foreign_wall_hg(w.fb, fmax, j, f ? s.Ag : s.Ah, G.aplane, q,
+                                                             Fs + f * 9 * fmax, true);
     }
     __syncthreads();
 }
@@ -1079,7 +1160,7 @@ __device__ __forceinline__ void fill_c_body(const DevState& s, int w, int q, int
         fill_phase(
             s, q, nbis, &s_next,
             [&](int k, int n, const NbInfo& nbi) {
-                foreign_c<N>(s, frn_c_of(s, k), nbi.nf[q], nbi.lev[0] - 1 >= lmin, Fs);
+                foreign_c<N>(s, {frn_c_of(s, k), nbi.nf[q], nbi.nd, nbi.lev[0] - 1 >= lmin}, Fs);
                 if (nbi.wait[q]) {
                     fill_ring_c<N>(s, G, k, n, w, 1, Fs);
                     wait_coarse(s, q, nbi);
@@ -1098,7 +1179,7 @@ __device__ __forceinline__ void fill_c_body(const DevState& s, int w, int q, int
                 item_rec_stage(s, c, q, srec[0]);
                 __syncthreads();
                 const ItemRec r = item_rec_of(srec[0]);
-                foreign_c<N>(s, frn_c_of(s, c), r.nf, true, Fs);
+                foreign_c<N>(s, {frn_c_of(s, c), r.nf, r.nd, true}, Fs);
                 fast_ring_c<N>(s, G, ((w == 2) ? s.plan_c2 : s.plan_c1) + (size_t)c * R * PLAN_INTS,
                                R, w, r, Fs, nullptr, true);
                 if (r.w3 || r.w4) wall_c_rows<N>(s, G, r.n, w, r.w3, r.w4, nullptr);
@@ -1161,7 +1242,7 @@ __device__ __forceinline__ void fill_c_body(const DevState& s, int w, int q, int
         double* T = tiles + st * SD;
         if (fast) {  // the ring, then Symmetric_C(2)_3/4, on the tile (and in memory if wr)
             const int* P = plans + st * PS;
-            foreign_c<N>(s, P + PLAN_INTS * R, r.nf, true, Fs);
+            foreign_c<N>(s, {P + PLAN_INTS * R, r.nf, r.nd, true}, Fs);
             fast_ring_c<N>(s, G, P, R, w, r, Fs, T, wr != 0);
             if (r.w3 || r.w4) {
                 wall_c_rows<N>(s, G, n, w, r.w3, r.w4, T, wr != 0);
@@ -1291,11 +1372,11 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, const Geo
             auto landed = [&]() { return !__syncthreads_or(mbar_wait(&bar[0], phase & 1u) ? 0 : 1); };
             bool ok;
             if (wr) {  // the whole ring, also to memory
-                foreign_hg<N>(s, G, Ps + PLAN_INTS * RG, r.nf, true, Fs);
+                foreign_hg<N>(s, G, {Ps + PLAN_INTS * RG, r.nf, r.nd, true}, Fs);
                 ok = landed();
                 if (ok) fast_ring_hg<N>(s, G, Ps, r, Fs, As);
             } else {
-                foreign_stream<N>(s, G, Ps + PLAN_INTS * RG, r.nf, nj, Fs);
+                foreign_stream<N>(s, G, {Ps + PLAN_INTS * RG, r.nf, r.nd, true}, nj, Fs);
                 ok = stream_ring<N>(s, G, Ps, r, nj, Fs, As, landed);
             }
             if (!ok) {
@@ -1327,7 +1408,8 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, const Geo
     fill_phase(
         s, q, nbis, &s_next,
         [&](int k, int n, const NbInfo& nbi) {
-            foreign_hg<N>(s, G, frn_hg_of(s, k), nbi.nf[q], nbi.lev[0] - 1 >= lmin, Fs);
+            foreign_hg<N>(s, G, {frn_hg_of(s, k), nbi.nf[q], nbi.nd, nbi.lev[0] - 1 >= lmin},
+                          Fs);
             if (nbi.wait[q]) {
                 fill_ring_hg<N>(s, G, k, n, 1, Fs);
                 wait_coarse(s, q, nbi);
@@ -1606,6 +1688,8 @@ void launch_fill_hg_stream(const DevState& s, const LaunchCfg& lc, cudaStream_t 
 #undef C_
     count_launches(1);
 }
+
+int foreign_slots(int nx, int ny) { return foreign_max(nx, ny); }
 
 void launch_build_plans(const DevState& s, const LaunchCfg& lc, cudaStream_t st) {
 #define C_(N) k_build_plans<N><<<lc.num_sms * 8, 128, 9 * sizeof(int) * ring1_len(s.nx, s.ny), st>>>(s)

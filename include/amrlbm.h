@@ -143,8 +143,9 @@ int amrlbm_set_launch(amrlbm_ctx* ctx, int32_t ctas_per_sm);
 /* Whether the current mesh's ghost fills need level order (1) or not (0):
  * [0] Fill_Ghost_Cells_C2, [1] Fill_Ghost_Cells_C, [2] Fill_Ghost_Cells_hg.
  * A fill needs it where a coarse-to-fine stencil reads a coarser
- * neighbour's ghost cell that is itself coarse-to-fine or a wall cell (the
- * reference's DO L = LevelMin, LevelMax loops, Fill_Ghost_Cells_C.f90:8-38);
+ * neighbour's ghost cell that is itself coarse-to-fine, or one behind a wall
+ * beside such a cell (the reference's DO L = LevelMin, LevelMax loops,
+ * Fill_Ghost_Cells_C.f90:8-38);
  * its kernels then take the leaves in level order with bounded waits. A
  * performance diagnostic; no counterpart in the reference. */
 int amrlbm_get_fill_order(amrlbm_ctx* ctx, int32_t needs_order[3]);
