@@ -656,10 +656,17 @@ __device__ void hg_item(const DevState& s, const Geo<N>& G, int k, const ItemRec
     constexpr int AP = (N + 2) * (N + 2), FP = 9 * AP;
     const int t = threadIdx.x, n = r.n, RG = ring1_len(N, N), fmax = s.fmax;
     const MpState& m = s.mp;
+    // the populations to evaluate of a ghost cell in direction d: those that
+    // streaming reads, three with Perfect_Shift_AMR and six with Lax-Wendroff
+    // (digits of stream_pops), or all nine where the ring goes to memory or is
+    // rounded as a whole (behind a wall)
+    const int nj = (!fast || wr) ? 9 : (r.dx == 1 ? 3 : 6), n1 = r.nf - r.nd, nk = n1 ? 9 : nj;
+    auto pop = [](int nn, int d, int k) { return nn == 9 ? k + 1 : (int)(stream_pops(d) >> (4 * k)) & 15; };
     // foreign cells: one thread per (slot, field and population)
-    for (int idx = t; idx < 18 * r.nd; idx += blockDim.x) {
-        const int j = idx % r.nd, fq = idx / r.nd, f = fq / 9, q = fq % 9 + 1;
-        const int meta = fb[j];
+    for (int idx = t; idx < 2 * nk * r.nd; idx += blockDim.x) {
+        const int j = idx % r.nd, fk = idx / r.nd, f = fk >= nk;
+        const int meta = fb[j], q = pop(nk, meta >> 8, f ? fk - nk : fk);
+        if (!q) continue;
         float v;
         if (plan_kind(meta) == 1) {
             v = dec_a<N, FMT>(m, G, f, (unsigned)fb[fmax + j], q);
@@ -669,12 +676,11 @@ __device__ void hg_item(const DevState& s, const Geo<N>& G, int k, const ItemRec
             for (int i = 0; i < 9; ++i) gg[i] = dec_a<N, FMT>(m, G, f, (unsigned)fb[(1 + i) * fmax + j], q);
             v = combine_f(meta, gg);
         }
-        Fs[fq * fmax + j] = v;
+        Fs[(f * 9 + q - 1) * fmax + j] = v;
     }
     __syncthreads();
     // those behind a wall (Bounce_Back_3/4, BC_Cell.f90:2-42), rounded as the
     // neighbour's ring in memory is: one thread per (slot, field)
-    const int n1 = r.nf - r.nd;
     if (n1) {
         for (int idx = t; idx < 2 * n1; idx += blockDim.x) {
             const int j = r.nd + idx % n1, f = idx / n1;
@@ -703,7 +709,7 @@ __device__ void hg_item(const DevState& s, const Geo<N>& G, int k, const ItemRec
     // the ring: copies per (cell, field), interpolated cells per (cell, population),
     // populations fastest, so that a cell's 9 threads share each source's rest load
     const int nC = 2 * r.na, nI = r.n2 + r.n3;
-    for (int u = t; u < nC + 9 * nI; u += blockDim.x) {
+    for (int u = t; u < nC + nj * nI; u += blockDim.x) {
         if (u < nC) {
             const int e = u % r.na, f = u / r.na;
             const int meta = pl[e];
@@ -713,16 +719,37 @@ __device__ void hg_item(const DevState& s, const Geo<N>& G, int k, const ItemRec
             }
             int xx, yy;
             ring1_xy(meta >> 8, N, N, xx, yy);
-            float v[9];
-            dec_a9<N, FMT>(m, G, f, (unsigned)pl[RG + e], v);
+            float* A = As + f * FP + yy * (N + 2) + xx;
+            if (nj == 9) {
+                float v[9];
+                dec_a9<N, FMT>(m, G, f, (unsigned)pl[RG + e], v);
 #pragma unroll
-            for (int q = 0; q < 9; ++q) As[f * FP + q * AP + yy * (N + 2) + xx] = v[q];
+                for (int q = 0; q < 9; ++q) A[q * AP] = v[q];
+            } else {
+                const unsigned off = (unsigned)pl[RG + e], pops = stream_pops(ghost_dir(xx, yy, N, N));
+                const float rest = __ldg((f ? m.A1g : m.A1h) + a_rest(G, off));
+                const unsigned short* D = (f ? m.Adg : m.Adh) + off;
+                const float is = f ? m.isg : m.ish;
+                unsigned short w[6];
+#pragma unroll
+                for (int k = 0; k < 6; ++k) {
+                    const int q = (int)(pops >> (4 * k)) & 15;
+                    if (k < nj && q) w[k] = __ldg(D + (unsigned)(q - 1) * G.aplane);
+                }
+#pragma unroll
+                for (int k = 0; k < 6; ++k) {
+                    const int q = (int)(pops >> (4 * k)) & 15;
+                    if (k < nj && q) A[(q - 1) * AP] = dec<FMT>(w[k]) * is + rq(q) * rest;
+                }
+            }
         } else {
-            const int v2 = u - nC, e = r.na + v2 / 9, q = v2 % 9 + 1;
+            const int v2 = u - nC, e = r.na + v2 / nj;
             const int meta = pl[e];
             const int kind = plan_kind(meta);
             int xx, yy;
             ring1_xy(meta >> 8, N, N, xx, yy);
+            const int q = pop(nj, ghost_dir(xx, yy, N, N), v2 % nj);
+            if (!q) continue;
             unsigned wd[9];
 #pragma unroll
             for (int i = 0; i < 9; ++i) wd[i] = (unsigned)pl[(1 + i) * RG + e];
@@ -776,7 +803,7 @@ __device__ void hg_item(const DevState& s, const Geo<N>& G, int k, const ItemRec
     }
     {
         const int x = t % N + 1, y = t / N + 1;
-        const float cfl = 1.f / (float)__ldg(s.dx + n);
+        const float cfl = 1.f / (float)r.dx;
         const bool shift = cfl > 0.9f;
         const float cA = cfl * 0.5f * (1.f + cfl), cC = cfl * 0.5f * (1.f - cfl);
         double csum = 0.0;  // C = sum of h, in FP64, rounded to FP32 at random
