@@ -7,12 +7,11 @@
 // in the reference, which flags blocks from the current field only
 // (Err_Interface, Refine_Derefine.f90:327-351).
 //
-// Every contraction is one kernel: C = A B with BF16 operands and FP32
-// accumulation on the tensor cores (mma.sync m16n8k16), A and B addressed
-// through strides so that transposes cost nothing. A convolution is an
-// im2col copy followed by that product; its backward pass is two more
-// products (dW = colT dY, dcol = dY WT) and a col2im gather. Weights are
-// kept in FP32 (Adam) and rounded to BF16 for every product.
+// Forward pass and gradient run one CTA per sample with everything of a
+// sample in shared memory (k_net): the convolutions as implicit products on
+// the tensor cores (mma.sync m16n8k16, BF16 operands, FP32 accumulation); the
+// weight gradients are products over the rows it leaves in memory (k_dw).
+// Weights are kept in FP32 (Adam) and rounded to BF16 for every product.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -24,17 +23,14 @@
 #include <vector>
 
 #include "amrlbm.h"
+#include "amrlbm_conv.cuh"
 #include "amrlbm_dev.cuh"
 #include "amrlbm_launch.h"
 
 namespace {
 
-constexpr int CH = 32;        // channels of every hidden layer
-constexpr int CIN = AMRLBM_NET_CHANNELS;
-constexpr int TILE = AMRLBM_NET_TILE;  // 18
-constexpr int PIX = TILE * TILE;       // 324
-constexpr int K1 = CIN * 9, K1P = (K1 + 15) / 16 * 16;  // 36 -> 48
-constexpr int K2 = CH * 9;                               // 288
+static_assert(CIN == AMRLBM_NET_CHANNELS && TILE == AMRLBM_NET_TILE, "sample layout");
+constexpr int K1 = CIN * 9;
 // FP32 parameter vector: W1 [K1][CH], b1, W2 [K2][CH], b2, W3 [K2][CH], b3, wd [CH], bd
 constexpr int O_W1 = 0, O_B1 = O_W1 + K1 * CH, O_W2 = O_B1 + CH, O_B2 = O_W2 + K2 * CH,
               O_W3 = O_B2 + CH, O_B3 = O_W3 + K2 * CH, O_WD = O_B3 + CH, O_BD = O_WD + CH,
@@ -119,130 +115,438 @@ void gemm(cudaStream_t st, int M, int N, int K, const __nv_bfloat16* A, long lon
 inline int blocks_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 8192); }
 #define GRID_STRIDE(i, n) for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (n); i += (long long)gridDim.x * blockDim.x)
 
-// input [n][CIN][TILE][TILE] (FP32) -> channels-last BF16 [n*PIX][CIN]
-__global__ void k_input(int n, const float* x, __nv_bfloat16* a) {
-    GRID_STRIDE(i, (long long)n * PIX * CIN) {
-        const long long row = i / CIN;
-        const int c = (int)(i % CIN), b = (int)(row / PIX), p = (int)(row % PIX);
-        a[i] = __float2bfloat16(x[((long long)b * CIN + c) * PIX + p]);
-    }
+// ---- forward pass and gradient, one CTA per sample ------------------------------
+struct GradSmem {
+    ConvSmem c;
+    __nv_bfloat16 wb[2][CH][KW2];  // [layer 2 | 3][ci][o * CH + co] = W[o * CH + ci][co]
+    __nv_bfloat16 dz[PIX][AROW];   // gradient of layer 3's pre-activations
+    int parg[NWARP][CH], arg[CH];
+    float dz3[CH];
+};
+// what a batch's weight gradients are formed from, BF16, rows = pixels of all
+// samples: the inputs of the three layers and the gradients of their
+// pre-activations
+struct GradRows {
+    __nv_bfloat16 *x0, *a1, *a2;        // [rows][CIN], [rows][CH] x 2
+    __nv_bfloat16* dz[3];               // [rows][CH]
+    float* df[3];                       // the same in FP32, for the bias gradients
+    float *pooled, *dlogit;             // [samples][CH], [samples]
+};
+
+__device__ __forceinline__ void ldsm4t(unsigned addr, unsigned* r) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
 }
-// im2col of a channels-last activation [n*PIX][cin]: col[row][k], k = o*cin + ci
-// (tap-major: the 16 columns of one product step are whole taps of adjacent
-// channels), o = (dy+1)*3 + (dx+1), zero outside the tile and for k >= cin*9
-__global__ void k_im2col(int n, int cin, int kp, const __nv_bfloat16* a, __nv_bfloat16* col) {
-    GRID_STRIDE(i, (long long)n * PIX * kp) {
-        const long long row = i / kp;
-        const int k = (int)(i % kp), b = (int)(row / PIX), p = (int)(row % PIX);
-        __nv_bfloat16 v = __float2bfloat16(0.f);
-        if (k < cin * 9) {
-            const int o = k / cin, ci = k % cin, y = p / TILE + o / 3 - 1, x = p % TILE + o % 3 - 1;
-            if (x >= 0 && x < TILE && y >= 0 && y < TILE)
-                v = a[((long long)b * PIX + y * TILE + x) * cin + ci];
+__device__ __forceinline__ void mma16816(float* d, const unsigned* a, unsigned b0, unsigned b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
+        "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// bit o: tap o of pixel p lies in the tile (0 for p outside it)
+__device__ __forceinline__ unsigned tap_mask(int p) {
+    if (p >= PIX) return 0u;
+    const int y = p / TILE, x = p % TILE;
+    const unsigned rows = (y > 0 ? 7u : 0u) | 7u << 3 | (y < TILE - 1 ? 7u << 6 : 0u);
+    const unsigned cols = (x > 0 ? 0111u : 0u) | 0222u | (x < TILE - 1 ? 0444u : 0u);
+    return rows & cols;
+}
+__device__ __forceinline__ int tap_shift(int o) { return (o / 3 - 1) * TILE + (o % 3 - 1); }
+
+// The transposed convolution of dz with W (wb[ci][o * CH + co]): the product of
+// each tap on its own, then their sum in tap order (acc), as a product with
+// all of W^T followed by the sum over the taps forms it. Operands as conv32's.
+__device__ __forceinline__ void conv32_back(const __nv_bfloat16 (*dz)[AROW], const __nv_bfloat16 (*wb)[KW2],
+                                            unsigned zero_row, int warp, int lane, float acc[3][4][4]) {
+    int pix[3];
+    unsigned vmask[3];
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+        pix[u] = 16 * (warp + NWARP * u) + (lane & 15);
+        vmask[u] = tap_mask(pix[u]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[u][j][i] = 0.f;
+    }
+    const unsigned abase = smem_addr(&dz[0][0]) + (unsigned)((lane >> 4) * 8 * 2);
+    const unsigned bbase = smem_addr(&wb[(lane & 7) + ((lane >> 4) << 3)][((lane >> 3) & 1) * 8]);
+    const bool third = warp + 2 * NWARP < MTILES;
+#pragma unroll 1
+    for (int o = 0; o < 9; ++o) {
+        unsigned b[2][8];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const unsigned at = bbase + (unsigned)((o * CH + 16 * c) * 2);
+            ldsm4(at, b[c][0], b[c][1], b[c][2], b[c][3]);
+            ldsm4(at + (unsigned)(16 * KW2 * 2), b[c][4], b[c][5], b[c][6], b[c][7]);
         }
-        col[i] = v;
+        const int shift = tap_shift(8 - o);  // pixel p - tap o
+#pragma unroll
+        for (int u = 0; u < 3; ++u) {
+            if (u == 2 && !third) break;
+            const bool in = (vmask[u] >> (8 - o)) & 1u;
+            float s[4][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s[j][i] = 0.f;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                unsigned a[4];
+                ldsm4(in ? abase + (unsigned)(((pix[u] + shift) * AROW + 16 * c) * 2) : zero_row, a[0], a[1],
+                      a[2], a[3]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) mma16816(s[j], a, b[c][2 * j], b[c][2 * j + 1]);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[u][j][i] = acc[u][j][i] + s[j][i];
+        }
     }
 }
-// z [m][CH] + bias -> ReLU: activation in FP32 and BF16
-__global__ void k_bias_relu(long long m, const float* z, const float* bias, float* af,
-                            __nv_bfloat16* ab) {
-    GRID_STRIDE(i, m * CH) {
-        const float v = fmaxf(z[i] + bias[i % CH], 0.f);
-        af[i] = v;
-        ab[i] = __float2bfloat16(v);
-    }
-}
-// global max pool of the last activation [n*PIX][CH] -> pooled [n][CH], argmax
-__global__ void k_maxpool(int n, const float* a, float* pooled, int* arg) {
-    GRID_STRIDE(i, (long long)n * CH) {
-        const int b = (int)(i / CH), c = (int)(i % CH);
-        float m = -1.f;
-        int am = 0;
-        for (int p = 0; p < PIX; ++p) {
-            const float v = a[((long long)b * PIX + p) * CH + c];
-            if (v > m) {
-                m = v;
-                am = p;
+
+// Logits of samples x [n][CIN][TILE][TILE]; with GRAD also the loss terms and
+// the rows that the gradients are summed from (k_dw, k_head_back).
+// The gradients equal, bit for bit, those of the plain sequence of products and
+// elementwise kernels that this replaced (im2col, product, bias and ReLU;
+// backwards product, col2im): the same operands in the same order.
+// What bounds it: some 5,000 mma.sync per sample with the ldmatrix that feed
+// them, 8 warps per CTA; one CTA per SM for the gradient (175 KB of shared
+// memory), two for the forward pass. The im2col matrices of that sequence,
+// 191 MB per layer for 512 samples, took 1.7 ms per gradient.
+template <bool GRAD>
+__global__ void __launch_bounds__(NT, GRAD ? 1 : 2)
+    k_net(const ForecastNet net, int n, const float* x, const float* y, float posw, float* logits,
+          float* lterm, GradRows rows) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    GradSmem& B = *reinterpret_cast<GradSmem*>(smraw);
+    ConvSmem& S = B.c;  // the forward pass has no more than this
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, g = lane >> 2, q = lane & 3;
+    load_weights(net, S, t);
+    __syncthreads();
+    if (GRAD)
+        for (int i = t; i < K2 * CH; i += NT) {
+            const int ci = i / K2, k = i % K2, o = k / CH, co = k % CH;
+            B.wb[0][ci][k] = S.w2[co][o * CH + ci];
+            B.wb[1][ci][k] = S.w3[co][o * CH + ci];
+        }
+    const unsigned zero_row = smem_addr(S.zero);
+    // rows of an activation to memory
+    auto put_rows = [&](const __nv_bfloat16 (*src)[AROW], __nv_bfloat16* dst) {
+        for (int i = t; i < PIX * (CH / 8); i += NT)
+            reinterpret_cast<uint4*>(dst)[i] =
+                *reinterpret_cast<const uint4*>(&src[i / (CH / 8)][i % (CH / 8) * 8]);
+    };
+    for (int b = blockIdx.x; b < n; b += gridDim.x) {
+        __syncthreads();  // the previous sample's buffers have been read
+        const float* xb = x + (size_t)b * CIN * PIX;
+        for (int p = t; p < PIX; p += NT) {
+            unsigned* x32 = reinterpret_cast<unsigned*>(&S.x0[p][0]);
+            x32[0] = pack2(__ldg(xb + p), __ldg(xb + PIX + p));
+            x32[1] = pack2(__ldg(xb + 2 * PIX + p), __ldg(xb + 3 * PIX + p));
+        }
+        __syncthreads();
+        two_layers(S, zero_row, warp, lane);
+        // layer 3 reduced to the channel maxima and the first pixel of each
+        float mx[4][2];
+        int am[4][2];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                mx[j][h] = -1.f;
+                am[j][h] = 0;
+            }
+        {
+            float acc[3][4][4];
+            conv32<KW2>(S.act[1], S.w3, zero_row, warp, lane, acc);
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+                const int mt = warp + NWARP * u;
+                if (mt >= MTILES) continue;
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const int p = 16 * mt + g + 8 * r;
+                    if (p >= PIX) continue;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const float v = fmaxf(acc[u][j][2 * r + h] + S.b[2][8 * j + 2 * q + h], 0.f);
+                            if (v > mx[j][h]) {
+                                mx[j][h] = v;
+                                am[j][h] = p;
+                            }
+                        }
+                }
             }
         }
-        pooled[i] = m;
-        arg[i] = am;
-    }
-}
-// dense output and the weighted binary cross-entropy on logits: logits[b],
-// dlogit[b] = w (sigmoid(z) - y) / n, loss terms lterm[b]
-__global__ void k_head(int n, const float* pooled, const float* w, const float* y, float posw,
-                       float* logits, float* dlogit, float* lterm) {
-    GRID_STRIDE(b, n) {
-        float z = w[O_BD - O_WD];
-        for (int c = 0; c < CH; ++c) z += w[c] * pooled[b * CH + c];
-        logits[b] = z;
-        if (y) {
-            const float yy = y[b], wt = yy > 0.5f ? posw : 1.f;
-            // log(1 + exp(-|z|)) + max(z, 0) - z y
-            const float l = log1pf(expf(-fabsf(z))) + fmaxf(z, 0.f) - z * yy;
-            lterm[b] = wt * l;
-            dlogit[b] = wt * (1.f / (1.f + expf(-z)) - yy) / (float)n;
+        // across the lanes of a column, then the warps: ties to the lower pixel
+        auto take = [](float& m, int& a, float m2, int a2) {
+            if (m2 > m || (m2 == m && a2 < a)) {
+                m = m2;
+                a = a2;
+            }
+        };
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int o = 4; o < 32; o <<= 1) {
+                    const float m2 = __shfl_xor_sync(0xffffffffu, mx[j][h], o);
+                    const int a2 = __shfl_xor_sync(0xffffffffu, am[j][h], o);
+                    take(mx[j][h], am[j][h], m2, a2);
+                }
+        if (g == 0)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    S.pmax[warp][8 * j + 2 * q + h] = mx[j][h];
+                    if (GRAD) B.parg[warp][8 * j + 2 * q + h] = am[j][h];
+                }
+        __syncthreads();
+        if (warp == 0) {
+            float p = S.pmax[0][lane];
+            int a = GRAD ? B.parg[0][lane] : 0;
+            for (int w = 1; w < NWARP; ++w) {
+                if (GRAD)
+                    take(p, a, S.pmax[w][lane], B.parg[w][lane]);
+                else
+                    p = fmaxf(p, S.pmax[w][lane]);
+            }
+            // the dense output, in channel order
+            float z = S.bd;
+            for (int c = 0; c < CH; ++c) z += S.wd[c] * __shfl_sync(0xffffffffu, p, c);
+            if (lane == 0) logits[b] = z;
+            if (GRAD) {
+                // weighted binary cross-entropy on the logit:
+                // log(1 + exp(-|z|)) + max(z, 0) - z y
+                const float yy = y[b], wt = yy > 0.5f ? posw : 1.f;
+                const float dl = wt * (1.f / (1.f + expf(-z)) - yy) / (float)n;
+                if (lane == 0) lterm[b] = wt * (log1pf(expf(-fabsf(z))) + fmaxf(z, 0.f) - z * yy);
+                const float d3 = p > 0.f ? dl * S.wd[lane] : 0.f;  // at the maximum alone
+                rows.pooled[(size_t)b * CH + lane] = p;
+                if (lane == 0) rows.dlogit[b] = dl;
+                B.dz3[lane] = d3;
+                B.arg[lane] = a;
+            }
+        }
+        if constexpr (GRAD) {
+        const size_t row0 = (size_t)b * PIX;
+        put_rows(S.act[0], rows.a1 + row0 * CH);
+        put_rows(S.act[1], rows.a2 + row0 * CH);
+        for (int i = t; i < PIX; i += NT)
+            reinterpret_cast<uint2*>(rows.x0 + row0 * CIN)[i] = *reinterpret_cast<const uint2*>(&S.x0[i][0]);
+        __syncthreads();
+        // layer 3: the maxima's pixels alone
+        for (int p = warp; p < PIX; p += NWARP) {
+            const float v = B.arg[lane] == p ? B.dz3[lane] : 0.f;
+            B.dz[p][lane] = __float2bfloat16(v);
+            rows.df[2][(row0 + p) * CH + lane] = v;
+        }
+        __syncthreads();
+        put_rows(B.dz, rows.dz[2] + row0 * CH);
+        // layer 2, then layer 1: the transposed convolution of the layer
+        // above, through the ReLU, in FP32 to memory and as BF16 over the
+        // activation (each value read by its writer alone)
+        auto back = [&](const __nv_bfloat16 (*dz)[AROW], const __nv_bfloat16 (*wb)[KW2],
+                        __nv_bfloat16 (*act)[AROW], float* df) {
+            float acc[3][4][4];
+            conv32_back(dz, wb, zero_row, warp, lane, acc);
+#pragma unroll
+            for (int u = 0; u < 3; ++u) {
+                const int mt = warp + NWARP * u;
+                if (mt >= MTILES) continue;
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const int p = 16 * mt + g + 8 * r;
+                    if (p >= PIX) continue;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int c = 8 * j + 2 * q;
+                        unsigned* a32 = reinterpret_cast<unsigned*>(&act[p][c]);
+                        const unsigned w = *a32;
+                        float2 v;
+                        v.x = __uint_as_float(w << 16) > 0.f ? acc[u][j][2 * r] : 0.f;
+                        v.y = __uint_as_float(w & 0xffff0000u) > 0.f ? acc[u][j][2 * r + 1] : 0.f;
+                        *a32 = pack2(v.x, v.y);
+                        *reinterpret_cast<float2*>(df + (row0 + p) * CH + c) = v;
+                    }
+                }
+            }
+            __syncthreads();
+        };
+        back(B.dz, B.wb[1], S.act[1], rows.df[1]);
+        put_rows(S.act[1], rows.dz[1] + row0 * CH);
+        back(S.act[1], B.wb[0], S.act[0], rows.df[0]);
+        put_rows(S.act[0], rows.dz[0] + row0 * CH);
         }
     }
 }
-// dense backward: gradients of wd, bd (one CTA, fixed order) and dpooled
-__global__ void k_head_back(int n, const float* pooled, const float* w, const float* dlogit,
-                            float* dpooled, float* grad_wd) {
-    const int t = threadIdx.x;
-    if (t <= CH) {
-        float s = 0.f;
-        for (int b = 0; b < n; ++b) s += dlogit[b] * (t < CH ? pooled[b * CH + t] : 1.f);
-        grad_wd[t] = s;  // [CH] weights then the bias
-    }
-    for (long long i = t; i < (long long)n * CH; i += blockDim.x) dpooled[i] = dlogit[i / CH] * w[i % CH];
-}
-// max-pool backward into dA [n*PIX][CH] (zero elsewhere)
-__global__ void k_unpool(int n, const float* dpooled, const int* arg, float* dA) {
-    GRID_STRIDE(i, (long long)n * PIX * CH) dA[i] = 0.f;
-}
-__global__ void k_unpool2(int n, const float* dpooled, const int* arg, float* dA) {
-    GRID_STRIDE(i, (long long)n * CH) {
-        const int b = (int)(i / CH), c = (int)(i % CH);
-        dA[((long long)b * PIX + arg[i]) * CH + c] = dpooled[i];
-    }
-}
-// ReLU backward: dz = dA where A > 0, as BF16 for the products
-__global__ void k_relu_back(long long m, const float* dA, const float* A, float* dz,
-                            __nv_bfloat16* dzb) {
-    GRID_STRIDE(i, m * CH) {
-        const float v = A[i] > 0.f ? dA[i] : 0.f;
-        dz[i] = v;
-        dzb[i] = __float2bfloat16(v);
-    }
-}
-// bias gradient: column sums of dz [m][CH] (one CTA per channel, fixed order)
-__global__ void k_colsum(long long m, const float* dz, float* out) {
-    __shared__ float red[256];
-    const int c = blockIdx.x;
+
+// Bias gradients: column sums of df [rows][CH]. 256 partial sums per column, of
+// the rows t, t + 256, ..., then a binary tree over them. colsum forms 4 of
+// the partial sums of one layer, coalesced, in CTAs of k_dw's launch beside the
+// products, which leave half of the SMs idle; k_head_back forms the trees.
+constexpr int NPART = 256;
+__device__ __forceinline__ void colsum(unsigned rows, const GradRows& R, int job, float* part) {
+    const int c = threadIdx.x % CH, l = job / (NPART / 4), t = job % (NPART / 4) * 4 + threadIdx.x / CH;
+    if (threadIdx.x >= 4 * CH) return;
+    const float* dz = l == 0 ? R.df[0] : l == 1 ? R.df[1] : R.df[2];
     float s = 0.f;
-    for (long long r = threadIdx.x; r < m; r += blockDim.x) s += dz[r * CH + c];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+#pragma unroll 16
+    for (unsigned r = t; r < rows; r += NPART) s += dz[(size_t)r * CH + c];
+    part[((size_t)l * CH + c) * NPART + t] = s;
+}
+// CTAs 0..95: the tree of one layer's channel; CTA 96: the dense layer's
+// gradient, the samples in order
+__global__ void __launch_bounds__(NPART) k_head_back(int n, const GradRows R, const float* part, float* grad) {
+    __shared__ float sh[NPART * (CH + 1)];
+    const int t = threadIdx.x, col = blockIdx.x;
+    if (col < 3 * CH) {
+        sh[t] = part[(size_t)col * NPART + t];
+        __syncthreads();
+        for (int o = NPART / 2; o > 0; o >>= 1) {
+            if (t < o) sh[t] += sh[t + o];
+            __syncthreads();
+        }
+        const int off[3] = {O_B1, O_B2, O_B3};
+        if (t == 0) grad[off[col / CH] + col % CH] = sh[0];
+        return;
+    }
+    float s = 0.f;
+    for (int b0 = 0; b0 < n; b0 += NPART) {
+        const int cnt = min(NPART, n - b0);
+        for (int i = t; i < cnt * CH; i += NPART) sh[i / CH * (CH + 1) + i % CH] = R.pooled[(size_t)b0 * CH + i];
+        for (int i = t; i < cnt; i += NPART) sh[i * (CH + 1) + CH] = R.dlogit[b0 + i];
+        __syncthreads();
+        if (t <= CH)
+            for (int b = 0; b < cnt; ++b)
+                s += sh[b * (CH + 1) + CH] * (t < CH ? sh[b * (CH + 1) + t] : 1.f);
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[c] = red[0];
+    if (t <= CH) grad[O_WD + t] = s;
 }
-// col2im: dA[row q][ci] = sum over the 3x3 offsets o of dcol[row q - o][o*cin + ci]
-__global__ void k_col2im(int n, int cin, int kp, const float* dcol, float* dA) {
-    GRID_STRIDE(i, (long long)n * PIX * cin) {
-        const long long row = i / cin;
-        const int ci = (int)(i % cin), b = (int)(row / PIX), p = (int)(row % PIX);
-        const int y = p / TILE, x = p % TILE;
-        float s = 0.f;
-        for (int o = 0; o < 9; ++o) {
-            const int py = y - (o / 3 - 1), px = x - (o % 3 - 1);
-            if (px >= 0 && px < TILE && py >= 0 && py < TILE)
-                s += dcol[((long long)b * PIX + py * TILE + px) * kp + o * cin + ci];
+
+// ---- weight gradients -------------------------------------------------------------
+// dW[o * cin + ci][co] = sum over the rows r (pixels of all samples, in order)
+// of in[r + tap o][ci] dz[r][co]: 16 rows per mma.sync, one accumulation chain
+// per output over all rows, as the plain product of the two matrices forms it
+// (the chain's order is kept: the tensor core truncates as it accumulates, and
+// training multiplies a change of the sum some hundredfold over ten steps).
+// A job is 16 x 16 outputs (two warps, a chain each); 36 jobs each for layers 3
+// and 2 (tap, half of the inputs, half of the outputs) and 6 for layer 1 (four
+// taps of the 4 inputs), one CTA each: warps 2-4 copy rows with cp.async into
+// a ring of stages, warps 0-1 multiply. Bound by the chain, 10,368 dependent
+// mma.sync for 512 samples. The generic product kernel loaded its operands
+// element by element between the steps of the chain: 30.8 ms per layer; all
+// three take 0.37 ms together.
+constexpr int DW_ROWS = 192, DW_STAGES = 6, DW_PITCH = 24;  // row pitch 48 bytes: no bank conflicts
+constexpr int DW_JOBS = 78, DW_THREADS = 160;
+struct DwSmem {
+    __nv_bfloat16 a[DW_STAGES][DW_ROWS][DW_PITCH], b[DW_STAGES][DW_ROWS][DW_PITCH];
+};
+// BYTES from src, or zeros
+template <int BYTES>
+__device__ __forceinline__ void cp_async_or_zero(void* dst, const void* src, bool ok) {
+    if (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src),
+                     "r"(ok ? 16 : 0)
+                     : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_addr(dst)), "l"(src),
+                     "r"(ok ? 8 : 0)
+                     : "memory");
+}
+__global__ void __launch_bounds__(DW_THREADS) k_dw(int n, const GradRows R, float* g, float* part) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    DwSmem& S = *reinterpret_cast<DwSmem*>(smraw);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const unsigned rows = (unsigned)n * PIX;
+    if (blockIdx.x >= DW_JOBS) return colsum(rows, R, blockIdx.x - DW_JOBS, part);
+    const int job = blockIdx.x, layer = job < 36 ? 3 : (job < 72 ? 2 : 1);
+    const int jj = layer == 3 ? job : (layer == 2 ? job - 36 : job - 72);
+    const int nh = jj & 1, ch = (jj >> 1) & 1, o = layer == 1 ? jj >> 1 : jj >> 2;  // o: tap, or row tile
+    const __nv_bfloat16* in = layer == 3 ? R.a2 : R.a1;
+    const __nv_bfloat16* dz = (layer == 3 ? R.dz[2] : layer == 2 ? R.dz[1] : R.dz[0]) + 16 * nh;
+    const int stages = (int)((rows + DW_ROWS - 1) / DW_ROWS);
+    auto load = [&](int s) {  // warps 2-4: rows of stage s
+        const int buf = s % DW_STAGES;
+#pragma unroll
+        for (int i = t - 64; i < DW_ROWS; i += 96) {
+            const unsigned r = (unsigned)(s * DW_ROWS + i);
+            const bool ok = r < rows;
+            const unsigned taps = ok ? tap_mask((int)(r % PIX)) : 0u;
+            const __nv_bfloat16* bs = dz + (size_t)(ok ? r : 0u) * CH;
+            cp_async_or_zero<16>(&S.b[buf][i][0], bs, ok);
+            cp_async_or_zero<16>(&S.b[buf][i][8], bs + 8, ok);
+            if (layer > 1) {
+                const bool in_tile = (taps >> o) & 1u;
+                const __nv_bfloat16* as = in + (size_t)(in_tile ? r + tap_shift(o) : 0u) * CH + 16 * ch;
+                cp_async_or_zero<16>(&S.a[buf][i][0], as, in_tile);
+                cp_async_or_zero<16>(&S.a[buf][i][8], as + 8, in_tile);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int oo = 4 * o + k;
+                    const bool in_tile = oo < 9 && ((taps >> oo) & 1u);
+                    cp_async_or_zero<8>(&S.a[buf][i][4 * k],
+                                        R.x0 + (size_t)(in_tile ? r + tap_shift(oo) : 0u) * CIN, in_tile);
+                }
+            }
         }
-        dA[i] = s;
+    };
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    if (warp > 1)
+        for (int s = 0; s < DW_STAGES - 1; ++s) {
+            if (s < stages) load(s);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+    // the lane's row and column of a warp's operand tiles (ldmatrix.trans):
+    // 16 rows of 16 inputs, 32 rows (two steps) of 8 outputs
+    const unsigned arow = (unsigned)(((lane & 7) + ((lane >> 4) << 3)) * DW_PITCH + ((lane >> 3) & 1) * 8) * 2u;
+    const unsigned brow = (unsigned)(lane * DW_PITCH + (warp & 1) * 8) * 2u;
+    for (int s = 0; s < stages; ++s) {
+        if (warp > 1) asm volatile("cp.async.wait_group %0;" ::"n"(DW_STAGES - 2) : "memory");
+        __syncthreads();  // stage s has landed, stage s - 1 has been read
+        if (warp > 1) {
+            if (s + DW_STAGES - 1 < stages) load(s + DW_STAGES - 1);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            continue;
+        }
+        const unsigned abase = smem_addr(&S.a[s % DW_STAGES][0][0]) + arow;
+        const unsigned bbase = smem_addr(&S.b[s % DW_STAGES][0][0]) + brow;
+        // the operands of two steps ahead of the products, whose chain then
+        // waits for itself alone
+        unsigned a[2][2][4], b[2][4];
+        auto fetch = [&](int k) {  // steps k, k + 1
+            const int m = (k / 2) % 2;
+            ldsm4t(abase + (unsigned)(k * 16 * DW_PITCH * 2), a[m][0]);
+            ldsm4t(abase + (unsigned)((k + 1) * 16 * DW_PITCH * 2), a[m][1]);
+            ldsm4t(bbase + (unsigned)(k * 16 * DW_PITCH * 2), b[m]);
+        };
+        fetch(0);
+#pragma unroll
+        for (int k = 0; k < DW_ROWS / 16; k += 2) {
+            const int m = (k / 2) % 2;
+            if (k + 2 < DW_ROWS / 16) fetch(k + 2);
+            mma16816(acc, a[m][0], b[m][0], b[m][1]);
+            mma16816(acc, a[m][1], b[m][2], b[m][3]);
+        }
+    }
+    if (warp > 1) return;
+    const int k0 = layer == 1 ? 16 * o : o * CH + 16 * ch, kk = layer == 1 ? K1 : K2;
+    float* out = g + (layer == 3 ? O_W3 : layer == 2 ? O_W2 : O_W1) + 16 * nh + 8 * warp;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int k = k0 + (lane >> 2) + 8 * (i >> 1);
+        if (k < kk) out[k * CH + 2 * (lane & 3) + (i & 1)] = acc[i];
     }
 }
 // Adam on the FP32 parameters
@@ -288,15 +592,10 @@ struct amrlbm_net {
     std::vector<void*> allocs;
     float *p = nullptr, *g = nullptr, *m1 = nullptr, *m2 = nullptr;  // [NPARAM]
     __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
-    // per batch row buffers
-    float *x = nullptr, *y = nullptr;
-    __nv_bfloat16 *a0 = nullptr, *col1 = nullptr, *col2 = nullptr, *col3 = nullptr;
-    float *z = nullptr, *a1f = nullptr, *a2f = nullptr, *a3f = nullptr, *dA = nullptr, *dz = nullptr,
-          *dcol = nullptr;
-    __nv_bfloat16 *a1b = nullptr, *a2b = nullptr, *a3b = nullptr, *dzb = nullptr;
-    float *pooled = nullptr, *dpooled = nullptr, *logits = nullptr, *dlogit = nullptr,
-          *lterm = nullptr;
-    int* arg = nullptr;
+    // a batch's samples and labels, logits and loss terms; partial bias sums
+    float *x = nullptr, *y = nullptr, *logits = nullptr, *lterm = nullptr, *part = nullptr;
+    GradRows rows{};
+    int num_sms = 0;
     int steps = 0;
     std::string err;
 };
@@ -319,52 +618,35 @@ void repack(amrlbm_net* net) {
     count_launches(1);
 }
 
-// forward of n samples already in net->x; the last activation in a3f
-void forward(amrlbm_net* net, int n) {
-    cudaStream_t st = net->st;
-    const long long m = (long long)n * PIX;
-    k_input<<<blocks_for(m * CIN), 256, 0, st>>>(n, net->x, net->a0);
-    k_im2col<<<blocks_for(m * K1P), 256, 0, st>>>(n, CIN, K1P, net->a0, net->col1);
-    gemm(st, (int)m, CH, K1P, net->col1, K1P, 1, net->w1, CH, 1, net->z, CH);
-    k_bias_relu<<<blocks_for(m * CH), 256, 0, st>>>(m, net->z, net->p + O_B1, net->a1f, net->a1b);
-    k_im2col<<<blocks_for(m * K2), 256, 0, st>>>(n, CH, K2, net->a1b, net->col2);
-    gemm(st, (int)m, CH, K2, net->col2, K2, 1, net->w2, CH, 1, net->z, CH);
-    k_bias_relu<<<blocks_for(m * CH), 256, 0, st>>>(m, net->z, net->p + O_B2, net->a2f, net->a2b);
-    k_im2col<<<blocks_for(m * K2), 256, 0, st>>>(n, CH, K2, net->a2b, net->col3);
-    gemm(st, (int)m, CH, K2, net->col3, K2, 1, net->w3, CH, 1, net->z, CH);
-    k_bias_relu<<<blocks_for(m * CH), 256, 0, st>>>(m, net->z, net->p + O_B3, net->a3f, net->a3b);
-    k_maxpool<<<blocks_for((long long)n * CH), 256, 0, st>>>(n, net->a3f, net->pooled, net->arg);
-    count_launches(9);
+ForecastNet weights_of(const amrlbm_net* net) {
+    ForecastNet f;
+    f.w1 = net->w1;
+    f.w2 = net->w2;
+    f.w3 = net->w3;
+    f.b1 = net->p + O_B1;
+    f.b2 = net->p + O_B2;
+    f.b3 = net->p + O_B3;
+    f.wd = net->p + O_WD;
+    f.bd = net->p + O_BD;
+    return f;
 }
 
-// backward after forward with labels: gradients into net->g
-void backward(amrlbm_net* net, int n) {
-    cudaStream_t st = net->st;
-    const long long m = (long long)n * PIX;
-    k_head_back<<<1, 256, 0, st>>>(n, net->pooled, net->p + O_WD, net->dlogit, net->dpooled,
-                                   net->g + O_WD);
-    k_unpool<<<blocks_for(m * CH), 256, 0, st>>>(n, net->dpooled, net->arg, net->dA);
-    k_unpool2<<<blocks_for((long long)n * CH), 256, 0, st>>>(n, net->dpooled, net->arg, net->dA);
+// logits of n samples x (device memory)
+void forward(amrlbm_net* net, int n, const float* x) {
+    const int grid = std::min(n, 2 * net->num_sms);
+    k_net<false><<<grid, NT, sizeof(ConvSmem), net->st>>>(weights_of(net), n, x, nullptr, 1.f,
+                                                           net->logits, nullptr, net->rows);
+    count_launches(1);
+}
+
+// logits, loss terms and gradient (net->g) of the n samples of the batch
+void gradient(amrlbm_net* net, int n, float pos_weight) {
+    const int grid = std::min(n, net->num_sms);
+    k_net<true><<<grid, NT, sizeof(GradSmem), net->st>>>(weights_of(net), n, net->x, net->y, pos_weight,
+                                                          net->logits, net->lterm, net->rows);
+    k_dw<<<DW_JOBS + 3 * NPART / 4, DW_THREADS, sizeof(DwSmem), net->st>>>(n, net->rows, net->g, net->part);
+    k_head_back<<<3 * CH + 1, NPART, 0, net->st>>>(n, net->rows, net->part, net->g);
     count_launches(3);
-    // layer 3
-    const float* A[3] = {net->a1f, net->a2f, net->a3f};
-    const __nv_bfloat16* col[3] = {net->col1, net->col2, net->col3};
-    const __nv_bfloat16* W[3] = {net->w1, net->w2, net->w3};
-    const int kp[3] = {K1P, K2, K2}, kk[3] = {K1, K2, K2};
-    const int ow[3] = {O_W1, O_W2, O_W3}, ob[3] = {O_B1, O_B2, O_B3};
-    const int cin[3] = {CIN, CH, CH};
-    for (int l = 2; l >= 0; --l) {
-        k_relu_back<<<blocks_for(m * CH), 256, 0, st>>>(m, net->dA, A[l], net->dz, net->dzb);
-        k_colsum<<<CH, 256, 0, st>>>(m, net->dz, net->g + ob[l]);
-        count_launches(2);
-        // dW = col^T dz: M = kk, N = CH, K = m (row strides of col are kp)
-        gemm(st, kk[l], CH, (int)m, col[l], 1, kp[l], net->dzb, CH, 1, net->g + ow[l], CH);
-        if (l == 0) break;
-        // dcol = dz W^T: M = m, N = kp, K = CH
-        gemm(st, (int)m, kp[l], CH, net->dzb, CH, 1, W[l], 1, CH, net->dcol, kp[l]);
-        k_col2im<<<blocks_for(m * cin[l]), 256, 0, st>>>(n, cin[l], kp[l], net->dcol, net->dA);
-        count_launches(1);
-    }
 }
 
 int net_fail(amrlbm_net* net, int code, const std::string& m) {
@@ -386,18 +668,7 @@ int load_batch(amrlbm_net* net, int n, const float* x, const float* y) {
 
 }  // namespace
 
-ForecastNet net_forecast_params(const amrlbm_net* net) {
-    ForecastNet f;
-    f.w1 = net->w1;
-    f.w2 = net->w2;
-    f.w3 = net->w3;
-    f.b1 = net->p + O_B1;
-    f.b2 = net->p + O_B2;
-    f.b3 = net->p + O_B3;
-    f.wd = net->p + O_WD;
-    f.bd = net->p + O_BD;
-    return f;
-}
+ForecastNet net_forecast_params(const amrlbm_net* net) { return weights_of(net); }
 
 extern "C" {
 
@@ -411,7 +682,8 @@ int amrlbm_net_create(uint64_t seed, int32_t max_batch, amrlbm_net** out) {
     amrlbm_net* net = new amrlbm_net();
     net->max_n = max_batch;
     cudaError_t e = cudaStreamCreateWithFlags(&net->st, cudaStreamNonBlocking);
-    const size_t n = (size_t)max_batch, m = n * PIX;
+    const size_t n = (size_t)max_batch;
+    cudaDeviceGetAttribute(&net->num_sms, cudaDevAttrMultiProcessorCount, dev);
     net->p = nalloc<float>(net, NPARAM, &e);
     net->g = nalloc<float>(net, NPARAM, &e);
     net->m1 = nalloc<float>(net, NPARAM, &e);
@@ -421,27 +693,26 @@ int amrlbm_net_create(uint64_t seed, int32_t max_batch, amrlbm_net** out) {
     net->w3 = nalloc<__nv_bfloat16>(net, (size_t)K2 * CH, &e);
     net->x = nalloc<float>(net, n * CIN * PIX, &e);
     net->y = nalloc<float>(net, n, &e);
-    net->a0 = nalloc<__nv_bfloat16>(net, m * CIN, &e);
-    net->col1 = nalloc<__nv_bfloat16>(net, m * K1P, &e);
-    net->col2 = nalloc<__nv_bfloat16>(net, m * K2, &e);
-    net->col3 = nalloc<__nv_bfloat16>(net, m * K2, &e);
-    net->z = nalloc<float>(net, m * CH, &e);
-    net->a1f = nalloc<float>(net, m * CH, &e);
-    net->a2f = nalloc<float>(net, m * CH, &e);
-    net->a3f = nalloc<float>(net, m * CH, &e);
-    net->a1b = nalloc<__nv_bfloat16>(net, m * CH, &e);
-    net->a2b = nalloc<__nv_bfloat16>(net, m * CH, &e);
-    net->a3b = nalloc<__nv_bfloat16>(net, m * CH, &e);
-    net->dA = nalloc<float>(net, m * CH, &e);
-    net->dz = nalloc<float>(net, m * CH, &e);
-    net->dzb = nalloc<__nv_bfloat16>(net, m * CH, &e);
-    net->dcol = nalloc<float>(net, m * K2, &e);
-    net->pooled = nalloc<float>(net, n * CH, &e);
-    net->dpooled = nalloc<float>(net, n * CH, &e);
-    net->arg = nalloc<int>(net, n * CH, &e);
     net->logits = nalloc<float>(net, n, &e);
-    net->dlogit = nalloc<float>(net, n, &e);
     net->lterm = nalloc<float>(net, n, &e);
+    net->part = nalloc<float>(net, 3 * CH * (size_t)NPART, &e);
+    net->rows.x0 = nalloc<__nv_bfloat16>(net, n * PIX * CIN, &e);
+    net->rows.a1 = nalloc<__nv_bfloat16>(net, n * PIX * CH, &e);
+    net->rows.a2 = nalloc<__nv_bfloat16>(net, n * PIX * CH, &e);
+    for (int l = 0; l < 3; ++l) {
+        net->rows.dz[l] = nalloc<__nv_bfloat16>(net, n * PIX * CH, &e);
+        net->rows.df[l] = nalloc<float>(net, n * PIX * CH, &e);
+    }
+    net->rows.pooled = nalloc<float>(net, n * CH, &e);
+    net->rows.dlogit = nalloc<float>(net, n, &e);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_net<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(ConvSmem));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_net<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(GradSmem));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DwSmem));
     if (e != cudaSuccess) {
         amrlbm_net_destroy(net);
         return AMRLBM_ERR_CUDA;
@@ -495,10 +766,7 @@ int amrlbm_net_set(amrlbm_net* net, const float* params) {
 int amrlbm_net_forward(amrlbm_net* net, int32_t n, const float* x, float* logits) {
     if (!net || !logits) return AMRLBM_ERR_ARG;
     if (int r = load_batch(net, n, x, nullptr)) return r;
-    forward(net, n);
-    k_head<<<blocks_for(n), 256, 0, net->st>>>(n, net->pooled, net->p + O_WD, nullptr, 1.f,
-                                               net->logits, net->dlogit, net->lterm);
-    count_launches(1);
+    forward(net, n, net->x);
     NCK(cudaMemcpyAsync(logits, net->logits, sizeof(float) * n, cudaMemcpyDeviceToHost, net->st));
     NCK(cudaStreamSynchronize(net->st));
     return AMRLBM_OK;
@@ -511,12 +779,7 @@ int amrlbm_net_forward_device(amrlbm_net* net, int32_t n, const float* x_dev, fl
     const size_t per = (size_t)CIN * PIX;
     for (int i0 = 0; i0 < n; i0 += net->max_n) {
         const int b = std::min(net->max_n, n - i0);
-        NCK(cudaMemcpyAsync(net->x, x_dev + per * i0, sizeof(float) * per * b,
-                            cudaMemcpyDeviceToDevice, net->st));
-        forward(net, b);
-        k_head<<<blocks_for(b), 256, 0, net->st>>>(b, net->pooled, net->p + O_WD, nullptr, 1.f,
-                                                   net->logits, net->dlogit, net->lterm);
-        count_launches(1);
+        forward(net, b, x_dev + per * i0);
         NCK(cudaMemcpyAsync(logits + i0, net->logits, sizeof(float) * b, cudaMemcpyDeviceToHost, net->st));
     }
     NCK(cudaStreamSynchronize(net->st));
@@ -527,11 +790,7 @@ int amrlbm_net_gradient(amrlbm_net* net, int32_t n, const float* x, const float*
                         float pos_weight, float* loss, float* grad) {
     if (!net || !y || !loss) return AMRLBM_ERR_ARG;
     if (int r = load_batch(net, n, x, y)) return r;
-    forward(net, n);
-    k_head<<<blocks_for(n), 256, 0, net->st>>>(n, net->pooled, net->p + O_WD, net->y, pos_weight,
-                                               net->logits, net->dlogit, net->lterm);
-    count_launches(1);
-    backward(net, n);
+    gradient(net, n, pos_weight);
     std::vector<float> lt(n);
     NCK(cudaMemcpyAsync(lt.data(), net->lterm, sizeof(float) * n, cudaMemcpyDeviceToHost, net->st));
     if (grad) NCK(cudaMemcpyAsync(grad, net->g, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost, net->st));
