@@ -58,6 +58,32 @@ struct Div {
         bad |= (unsigned)((e - 63u > 1960u) & !a0);
         return a0 ? q : q1;
     }
+    // the same quotient up to the sign of a zero (a dividend -0 gives +0):
+    // without the select
+    __device__ __forceinline__ double quot(double a, double b, double yb) {
+        if (SAFE) return a / b;
+        const double q = a * yb;
+        const double q1 = __fma_rn(__fma_rn(-q, b, a), yb, q);
+        const unsigned h = (unsigned)__double2hiint(q) & 0x7fffffffu;
+        bad |= (unsigned)((h - 0x03f00000u > 0x7a800000u) & ((h | (unsigned)__double2loint(q)) != 0u));
+        return q1;
+    }
+    __device__ __forceinline__ double q3(double a) { return quot(a, 3.0, 1.0 / 3.0); }
+    __device__ __forceinline__ double q6(double a) { return quot(a, 6.0, 1.0 / 6.0); }
+    __device__ __forceinline__ double q12(double a) { return quot(a, 12.0, 1.0 / 12.0); }
+    __device__ __forceinline__ double q36(double a) { return quot(a, 36.0, 1.0 / 36.0); }
+    // a/3 for a dividend known to be 0 or within [2^-960, 2^1001)
+    __device__ __forceinline__ double n3(double a) {
+        if (SAFE) return a / 3.0;
+        const double q = a * (1.0 / 3.0);
+        return __fma_rn(__fma_rn(-q, 3.0, a), 1.0 / 3.0, q);
+    }
+    // sets bad unless 2^-e <= |a| < 2^e (low: the lower bound too)
+    __device__ __forceinline__ void within(double a, unsigned e, bool low) {
+        if (SAFE) return;
+        const unsigned x = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu;
+        bad |= (unsigned)(low ? x - (1023u - e) > 2u * e - 1u : x > 1023u + e - 1u);
+    }
     __device__ __forceinline__ double d3(double a) { return (*this)(a, 3.0, 1.0 / 3.0); }
     __device__ __forceinline__ double d6(double a) { return (*this)(a, 6.0, 1.0 / 6.0); }
     __device__ __forceinline__ double d12(double a) { return (*this)(a, 12.0, 1.0 / 12.0); }

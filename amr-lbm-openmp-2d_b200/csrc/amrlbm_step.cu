@@ -611,27 +611,23 @@ __device__ void wall_c(const DevState& s, const Geo<N>& G, int n, const NbInfo& 
 
 // ---------------------------------------------------------------------------
 // Collision_h_g_AMR (LBM_Subroutines.f90:116-189) of cell c of block n.
-// T: shared C block (G.c(0,..)); Hb, Gb: the block's post-streaming h and g
-// planes (plane stride nx*ny; staged in shared memory or in memory); unless
-// FUSED, P, Ux, Uy are read from memory, where nothing writes them during the
+// with IEEE divisions. T: shared C block (G.c(0,..)); the post-streaming h and
+// g planes are read from memory; unless FUSED, P, Ux, Uy are read from memory, where nothing writes them during the
 // launch. Writes the post-collision populations A to memory. FUSED: P, Ux,
 // Uy come from Macroscopic_Values_g_AMR (:205-240) evaluated here on the
 // same C ring.
 // BGK: the collision of g is BGK_Collision_AMR (LBM_Subroutines.f90:337-344,
 // g*(1-s9) + geq*s9) instead of MRT_Collision_AMR, the alternative the
 // reference leaves commented out at :180
-template <bool SAFE, bool FUSED, bool SHH, bool SHG, int N, bool BGK = false, bool BATCH = false>
-__device__ __forceinline__ unsigned collide_cell(const DevState& s, const Geo<N>& G, int n, int c,
-                                                 double inv_dx, const double* T, const double* Hb,
-                                                 const double* Gb) {
+template <bool FUSED, int N, bool BGK = false, bool BATCH = false>
+__device__ __forceinline__ void collide_ieee(const DevState& s, const Geo<N>& G, int n, int c,
+                                             double inv_dx, const double* T) {
     const PhysD& ph = phys_of<BATCH>(s, n);
     const int nx = G.nx, BP = G.bplane, PP = G.pplane;
     const double inv_dx2 = inv_dx * inv_dx;
-    const double* Hn = Hb + c;
-    const double* Gn = Gb + c;
-    auto ldh = [&](const double* p) { return SHH ? lds(p) : __ldg(p); };
-    auto ldp = [&](const double* p) { return SHG ? lds(p) : __ldg(p); };
-    Div<SAFE> dv;
+    const double* Hn = s.Bh + (size_t)n * 9 * BP + c;
+    const double* Gn = s.Bg + (size_t)n * 9 * BP + c;
+    Div<true> dv;
     {
         const int x = c % nx + 1, y = c / nx + 1;
         auto Cs = [&](int a, int b) { return T[G.c(0, x + a, y + b)]; };
@@ -664,7 +660,7 @@ __device__ __forceinline__ unsigned collide_cell(const DevState& s, const Geo<N>
             gradient_iso_f(dv, inv_dx, Cs, gx, gy);
             const double Fx = mu * gx;
             const double Fy = mu * gy + Fb;
-            auto g = [&](int k) { return ldp(Gn + (k - 1) * BP); };
+            auto g = [&](int k) { return __ldg(Gn + (k - 1) * BP); };
             const double sx = ((((g(2) - g(4)) + g(6)) - g(7)) - g(8)) + g(9);
             const double sy = ((((g(3) - g(5)) + g(6)) + g(7)) - g(8)) - g(9);
             const double rr = __drcp_rn(Rho);
@@ -704,21 +700,21 @@ __device__ __forceinline__ unsigned collide_cell(const DevState& s, const Geo<N>
             const double eN = (double)d_ex(k) * ni + (double)d_ey(k) * nj;
             const double Gm = wk * (1.0 + eU * (3.0 + 4.5 * eU) - U215);
             const double heq = c0 * (Gm + tmp * wk * eN);
-            s.Ah[G.a(n, k, x, y)] = ldh(Hn + (k - 1) * BP) * ph.omwc + heq * ph.wc;
+            s.Ah[G.a(n, k, x, y)] = __ldg(Hn + (k - 1) * BP) * ph.omwc + heq * ph.wc;
             const double Ak = (Gm - wk) * ph.dRho3 + Gm * mu;
             const double Bk = ((double)d_ey(k) - Uy) * Gm * Fb;
             const double hc = Ak * (Ec(k) - ud_c) + Bk;
             const double geq = P * wk + dv.d3((Gm - wk) * Rho) - 0.5 * hc;
             if (BGK)  // g(:)*(1.d0 - s9) + geq(:)*s9
-                f[k] = ldp(Gn + (k - 1) * BP) * (1.0 - s9) + geq * s9;
+                f[k] = __ldg(Gn + (k - 1) * BP) * (1.0 - s9) + geq * s9;
             else
-                f[k] = ldp(Gn + (k - 1) * BP) - geq;
+                f[k] = __ldg(Gn + (k - 1) * BP) - geq;
             hm[k] = Ak * (Em(k) - ud_m) + Bk;
         }
         if (BGK) {
 #pragma unroll
             for (int k = 1; k <= 9; ++k) s.Ag[G.a(n, k, x, y)] = f[k] + hm[k];
-            return dv.bad;
+            return;
         }
         // MRT_Collision_AMR (:348-361): Convert, relax 8 and 9, Reconvt, /36
         double m[10];
@@ -745,11 +741,188 @@ __device__ __forceinline__ unsigned collide_cell(const DevState& s, const Geo<N>
         o[9] = b2 + 6.0 * m[4] + 3.0 * m[5] - 6.0 * m[6] - 3.0 * m[7] - 9.0 * m[9];
 #pragma unroll
         for (int k = 1; k <= 9; ++k)
-            s.Ag[G.a(n, k, x, y)] = (ldp(Gn + (k - 1) * BP) - dv.d36(o[k])) + hm[k];
+            s.Ag[G.a(n, k, x, y)] = (__ldg(Gn + (k - 1) * BP) - dv.d36(o[k])) + hm[k];
     }
-    return dv.bad;
 }
 
+// The same collision, bit for bit (up to the sign of zeros), with about three
+// quarters of the FP64 operations: opposite directions share their terms
+// (Ec(-e) = -Ec(e), 4.5 eU, eU (3 +- 4.5 eU)), products by powers of two (0.5,
+// 2, 4, 1/dx) ride in exact FMAs, gradients are formed unscaled and scaled
+// once (1/dx is a power of two), and zero components of e drop out. Where that
+// is not exact (quotients outside their range, a non-finite velocity) dv.bad
+// is returned and the caller takes collide_ieee, which reads h and g from
+// memory. SMEM: the block's h and g planes Hb, Gb are staged in shared memory,
+// and each population h of this cell, once read, gives its place to hm (the
+// forcing of g), which is needed only at the end. Differences of C below
+// 2^-1000, where 1/dx times them is no longer exact, carry the reference's
+// rounding to within 2^-1070.
+// The consumer shares the CTA's time with the copies and the ghost fill, so
+// fewer operations gave 26.0 -> 25.4 us over 788 leaves of 16x16 cells and
+// 455 -> 450 us over 17,568; three CTAs per SM (80 registers, one stage) were
+// slower: 25.7 and 464 us.
+template <bool FUSED, bool SMEM, int N, bool BGK, bool BATCH>
+__device__ __forceinline__ unsigned collide_fast(const DevState& s, const Geo<N>& G, int n, int c,
+                                                 double inv_dx, const double* T, double* Hb,
+                                                 const double* Gb) {
+    const PhysD& ph = phys_of<BATCH>(s, n);
+    const int nx = G.nx, BP = G.bplane, PP = G.pplane;
+    double* Hn = Hb + c;
+    const double* Gn = Gb + c;
+    auto ldh = [&](int k) { return SMEM ? lds(Hn + (k - 1) * BP) : __ldg(Hn + (k - 1) * BP); };
+    auto ldg = [&](int k) { return SMEM ? lds(Gn + (k - 1) * BP) : __ldg(Gn + (k - 1) * BP); };
+    Div<false> dv;
+    const int x = c % nx + 1, y = c / nx + 1;
+    const double* Tc = T + G.c(0, x, y);
+    auto Cs = [&](int a, int b) { return lds(Tc + (b * G.cp + a)); };
+    const double c0 = Cs(0, 0);
+    const double hd = 0.5 * inv_dx, qd = 0.25 * inv_dx;
+    double D[4], mu, DcDx, DcDy, gx, gy;  // D: C(e) - C(-e) along directions 2, 3, 6, 7
+    {
+        const double E = Cs(1, 0), W = Cs(-1, 0), Nn = Cs(0, 1), S = Cs(0, -1);
+        const double NE = Cs(1, 1), SW = Cs(-1, -1), NW = Cs(-1, 1), SE = Cs(1, -1);
+        D[0] = E - W;
+        D[1] = Nn - S;
+        D[2] = NE - SW;
+        D[3] = NW - SE;
+        // Laplacian_AMR + Chemical_Potential_AMR (:94-112,316-333)
+        const double D2C = dv.q6(__fma_rn(4.0, ((S + W) + E) + Nn, ((SW + SE) + NW) + NE) - 20.0 * c0);
+        mu = __fma_rn(-(ph.kappa * D2C), inv_dx * inv_dx, ph.Beta4 * c0 * (c0 - 1.0) * (c0 - 0.5));
+        const double t1 = dv.q3(D[0]), t2 = dv.q3(D[1]);
+        // Gradient_ED_AMR of Ec (:281-289)
+        DcDx = hd * ((t1 + t1) + dv.q12(((D[2] - D[3]) + D[2]) - D[3]));
+        DcDy = hd * ((t2 + t2) + dv.q12(((D[2] + D[3]) + D[2]) + D[3]));
+        if (FUSED) {  // Gradient_AMR (:293-312)
+            gx = inv_dx * (t1 + dv.q12(((NE + SE) - NW) - SW));
+            gy = inv_dx * (t2 + dv.q12(((NE + NW) - SE) - SW));
+        }
+    }
+    const double Rho = ph.Rhol + c0 * ph.dRho;
+    const double Fb = (ph.Rhoh - Rho) * ph.Gy;
+    double P, Ux, Uy;
+    if (FUSED) {  // Macroscopic_Values_g_AMR (:205-240)
+        const double g2 = ldg(2), g3 = ldg(3), g4 = ldg(4), g5 = ldg(5), g6 = ldg(6), g7 = ldg(7),
+                     g8 = ldg(8), g9 = ldg(9);
+        const double sx = ((((g2 - g4) + g6) - g7) - g8) + g9;
+        const double sy = ((((g3 - g5) + g6) + g7) - g8) - g9;
+        const double rr = __drcp_rn(Rho);
+        Ux = dv(__fma_rn(0.5, mu * gx, 3.0 * sx), Rho, rr);
+        Uy = dv(__fma_rn(0.5, mu * gy + Fb, 3.0 * sy), Rho, rr);
+        P = (((((((ldg(1) + g2) + g3) + g4) + g5) + g6) + g7) + g8) + g9;
+        P = P + ph.dRho6 * (Ux * gx + Uy * gy);
+    } else {
+        P = __ldg(s.P + (size_t)n * PP + c);
+        Ux = __ldg(s.Ux + (size_t)n * PP + c);
+        Uy = __ldg(s.Uy + (size_t)n * PP + c);
+    }
+    const double U215 = 1.5 * (Ux * Ux + Uy * Uy);
+    dv.within(U215, 400, false);  // with Rho: (Gm - wk) Rho, 0 or at least 2^-59 Rho, is in n3's range
+    dv.within(Rho, 400, true);
+    const double ud_c = Ux * DcDx + Uy * DcDy;
+    // ED_M_AMR (:262-277) times 4 dx, along direction (a, b)
+    const double c3 = 3.0 * c0;
+    auto M = [&](int a, int b) { return (5.0 * Cs(a, b) - (Cs(-a, -b) + c3)) - Cs(2 * a, 2 * b); };
+    double ud_m;
+    {
+        const double m6 = M(1, 1), m7 = M(-1, 1), m8 = M(-1, -1), m9 = M(1, -1);
+        const double DmX = qd * (dv.q3(M(1, 0) - M(-1, 0)) + dv.q12(((m6 - m7) - m8) + m9));
+        const double DmY = qd * (dv.q3(M(0, 1) - M(0, -1)) + dv.q12(((m6 + m7) - m8) - m9));
+        ud_m = Ux * DmX + Uy * DmY;
+    }
+    double ni, nj;
+    {  // normal_AMR (:25-37)
+        const double t = sqrt(DcDx * DcDx + DcDy * DcDy + 1.e-32), rt = __drcp_rn(t);
+        ni = dv.quot(DcDx, t, rt);
+        nj = dv.quot(DcDy, t, rt);
+    }
+    const double tmp = dv.quot(12.0 * (1.0 - c0), ph.W, ph.yW) * ph.M0;
+    double s9;
+    {
+        double tau;
+        if (c0 < 0.0) {
+            tau = ph.taul5;
+        } else if (c0 > 1.0) {
+            tau = ph.tauh5;
+        } else {
+            tau = c0 * ph.itau_d + ph.itaul;
+            tau = __drcp_rn(tau) + 0.5;
+        }
+        s9 = __drcp_rn(tau);
+    }
+    double f[10], hmr[10];
+    // population k: G = Gamma_k, wk, (ey - Uy) b, tmp wk eN = q, Ec - ud_c, Em
+    auto one = [&](int k, double wk, double G_, double b, double q, double pw, double ec, double em) {
+        const double heq = c0 * (G_ + q);
+        s.Ah[G.a(n, k, x, y)] = ldh(k) * ph.omwc + heq * ph.wc;
+        const double dG = G_ - wk;
+        const double Ak = dG * ph.dRho3 + G_ * mu, Bk = b * G_ * Fb;
+        const double geq = __fma_rn(-0.5, Ak * ec + Bk, pw + dv.n3(dG * Rho));
+        f[k] = BGK ? ldg(k) * (1.0 - s9) + geq * s9 : ldg(k) - geq;
+        const double hm = Ak * __fma_rn(em, qd, -ud_m) + Bk;
+        if (SMEM)
+            Hn[(k - 1) * BP] = hm;
+        else
+            hmr[k] = hm;
+    };
+    {  // the rest population: e = 0, Ec = 0, Em = (-C - 3C) + 5C - C
+        const double wk = wa(1);
+        one(1, wk, wk * (1.0 - U215), -Uy, 0.0, P * wk, -ud_c, (5.0 * c0 - (c0 + c3)) - c0);
+    }
+    // direction i = (a, b) and the opposite one o: eU, eN of i
+    auto pair = [&](int i, int a, int b, double wk, double eU, double eN, double tw, double pw, double d) {
+        const int o = i + (i % 4 < 2 ? -2 : 2);
+        const double e45 = 4.5 * eU, q = tw * eN;
+        one(i, wk, wk * ((1.0 + eU * (3.0 + e45)) - U215), (double)b - Uy, q, pw, __fma_rn(d, hd, -ud_c), M(a, b));
+        one(o, wk, wk * ((1.0 - eU * (3.0 - e45)) - U215), (double)-b - Uy, -q, pw, __fma_rn(-d, hd, -ud_c),
+            M(-a, -b));
+    };
+    {
+        const double wk = wa(2), tw = tmp * wk, pw = P * wk;
+        pair(2, 1, 0, wk, Ux, ni, tw, pw, D[0]);
+        pair(3, 0, 1, wk, Uy, nj, tw, pw, D[1]);
+    }
+    {
+        const double wk = wa(6), tw = tmp * wk, pw = P * wk;
+        pair(6, 1, 1, wk, Ux + Uy, ni + nj, tw, pw, D[2]);
+        pair(7, -1, 1, wk, Uy - Ux, nj - ni, tw, pw, D[3]);
+    }
+    auto out = [&](int k, double v) {
+        s.Ag[G.a(n, k, x, y)] = v + (SMEM ? lds(Hn + (k - 1) * BP) : hmr[k]);
+    };
+    if (BGK) {
+#pragma unroll
+        for (int k = 1; k <= 9; ++k) out(k, f[k]);
+        return dv.bad;
+    }
+    // MRT_Collision_AMR (:348-361): Convert, relax 8 and 9, Reconvt, /36
+    const double S = f[6] + f[7] + f[8] + f[9], R = f[2] + f[3] + f[4] + f[5];
+    const double m1 = f[1] + f[2] + f[3] + f[4] + f[5] + f[6] + f[7] + f[8] + f[9];
+    const double m2 = __fma_rn(2.0, S, __fma_rn(-4.0, f[1], -f[2]) - f[3] - f[4] - f[5]);
+    const double m3 = __fma_rn(-2.0, R, 4.0 * f[1]) + f[6] + f[7] + f[8] + f[9];
+    const double f24 = f[2] - f[4], f35 = f[3] - f[5];
+    const double m4 = f24 + f[6] - f[7] - f[8] + f[9];
+    const double m5 = __fma_rn(-2.0, f24, f[6]) - f[7] - f[8] + f[9];
+    const double m6 = f35 + f[6] + f[7] - f[8] - f[9];
+    const double m7 = __fma_rn(-2.0, f35, f[6]) + f[7] - f[8] - f[9];
+    const double n8 = 9.0 * ((f[2] - f[3] + f[4] - f[5]) * s9);
+    const double n9 = 9.0 * ((f[6] - f[7] + f[8] - f[9]) * s9);
+    const double b1 = __fma_rn(-2.0, m3, __fma_rn(4.0, m1, -m2));
+    const double b2 = __fma_rn(2.0, m2, 4.0 * m1) + m3;
+    auto fin = [&](int k, double o) { out(k, ldg(k) - dv.q36(o)); };
+    fin(1, 4.0 * (m1 - m2 + m3));
+    const double p45 = 6.0 * (m4 - m5), p67 = 6.0 * (m6 - m7);
+    fin(2, b1 + p45 + n8);
+    fin(3, b1 + p67 - n8);
+    fin(4, b1 - p45 + n8);
+    fin(5, b1 - p67 - n8);
+    const double a4 = 6.0 * m4, a5 = 3.0 * m5, a6 = 6.0 * m6, a7 = 3.0 * m7;
+    const double e1 = b2 + a4 + a5, e2 = b2 - a4 - a5;
+    fin(6, e1 + a6 + a7 + n9);
+    fin(7, e2 + a6 + a7 - n9);
+    fin(8, e2 - a6 - a7 + n9);
+    fin(9, e1 - a6 - a7 - n9);
+    return dv.bad;
+}
 
 // Macroscopic_Values_g_AMR (LBM_Subroutines.f90:205-240) of cell c of block n
 // from T and the block's g planes Gb (shared memory or memory); dc = the
@@ -791,14 +964,14 @@ __device__ __forceinline__ unsigned macro_g_cell_f(const DevState& s, const Geo<
 }
 // Collision of every cell of block n: the branch-free exact division path,
 // and the IEEE path for a cell whose flag says a quotient left its range.
-// SHH, SHG: Hb, Gb point to shared memory (else to memory)
-template <int N, bool FUSED, bool SHH, bool SHG, bool BGK = false, bool BATCH = false>
+// SMEM: Hb, Gb point to shared memory (else to memory)
+template <int N, bool FUSED, bool SMEM, bool BGK = false, bool BATCH = false>
 __device__ __forceinline__ void collide_block(const DevState& s, const Geo<N>& G, int n, int dx,
-                                              const double* T, const double* Hb, const double* Gb) {
+                                              const double* T, double* Hb, const double* Gb) {
     const double inv_dx = 1.0 / (double)dx;  // dx is a power of two: exact
     for (int c = threadIdx.x; c < G.nx * G.ny; c += blockDim.x)
-        if (collide_cell<false, FUSED, SHH, SHG, N, BGK, BATCH>(s, G, n, c, inv_dx, T, Hb, Gb))
-            collide_cell<true, FUSED, SHH, SHG, N, BGK, BATCH>(s, G, n, c, inv_dx, T, Hb, Gb);
+        if (collide_fast<FUSED, SMEM, N, BGK, BATCH>(s, G, n, c, inv_dx, T, Hb, Gb))
+            collide_ieee<FUSED, N, BGK, BATCH>(s, G, n, c, inv_dx, T);
 }
 
 // Macroscopic_Values_g_AMR of every cell of block n; returns this thread's
@@ -1128,15 +1301,14 @@ __device__ __forceinline__ void fill_c_body(const DevState& s, int w, int q, int
     if (collide && blockIdx.x == 0 && t == 0)
         atomicAdd(&s.cnt->updates, (unsigned long long)total * (unsigned long long)(G.nx * G.ny));
     // stage st: C tile at tiles + st*SD, then h planes (if staged), then g planes
-    auto consume = [&](int n, int dx, const double* T) {
-        const double* Hs = stage_h(CONSUMER) ? T + G.cplane : s.Bh + (size_t)n * HP;
+    auto consume = [&](int n, int dx, double* T) {
+        double* Hs = stage_h(CONSUMER) ? T + G.cplane : s.Bh + (size_t)n * HP;
         const double* Gs = stage_g(CONSUMER) ? T + G.cplane + (stage_h(CONSUMER) ? HP : 0)
                                              : s.Bg + (size_t)n * HP;
         if (CONSUMER == CONS_MACRO_G)
             err_reduce(s, n, macro_g_block<N, true, BATCH>(s, G, n, dx, T, Gs), red);
         else if (CONSUMER != CONS_NONE)
-            collide_block<N, CONSUMER == CONS_COLLIDE_FUSED, stage_h(CONSUMER), stage_g(CONSUMER), BGK,
-                          BATCH>(s, G, n, dx, T, Hs, Gs);
+            collide_block<N, CONSUMER == CONS_COLLIDE_FUSED, true, BGK, BATCH>(s, G, n, dx, T, Hs, Gs);
     };
     const unsigned tb = (unsigned)G.cplane * 8, hb = (unsigned)HP * 8;
     auto copy_tile = [&](int st, int nn, int c) {  // thread 0: item c, block nn
@@ -1489,7 +1661,7 @@ __global__ void __launch_bounds__(256, 2) k_collide(DevState s) {
     for (int m = blockIdx.x; m < nleaf; m += gridDim.x) {
         const int n = s.leaf[m];
         load_tile_c<N>(s, G, n, T);
-        collide_block<N, false, false, false, BGK, BATCH>(s, G, n, __ldg(s.dx + n), T, s.Bh + (size_t)n * 9 * G.bplane,
+        collide_block<N, false, false, BGK, BATCH>(s, G, n, __ldg(s.dx + n), T, s.Bh + (size_t)n * 9 * G.bplane,
                                                    s.Bg + (size_t)n * 9 * G.bplane);
         __syncthreads();
     }
