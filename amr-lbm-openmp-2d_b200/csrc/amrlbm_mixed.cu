@@ -112,11 +112,6 @@ __device__ __forceinline__ float dec_a(const MpState& m, const Geo<N>& G, int f,
     return dec<FMT>(d) * (f ? m.isg : m.ish) + rq(q) * rest;
 }
 
-// generic-proxy writes of earlier launches seen by the bulk copies that read them
-__device__ __forceinline__ void fence_proxy_async_all() {
-    asm volatile("fence.proxy.async;" ::: "memory");
-}
-
 // ---- level order ----------------------------------------------------------
 // Fill q of a launch needs level order when a coarse-to-fine stencil reads a
 // coarser neighbour's ring cell that is not a foreign cell (fillinfo[q]):
@@ -554,8 +549,6 @@ __global__ void __launch_bounds__(N * N, (N == 16 ? 3 : 8)) k_mp_collide(const _
     // thread 0 copies item kk (block nn) into stage st
     auto issue = [&](int st, int kk, int nn) {
         unsigned char* S = stages + st * SL::BYTES;
-        fence_proxy_async_all();
-        fence_proxy_async();
         mbar_expect_tx(&bar[st], SL::BYTES);
         bulk_g2s(S, m.C + (size_t)nn * G.cplane, SL::TILE, &bar[st]);
         bulk_g2s(S + SL::O_DH, m.Bdh + (size_t)nn * 9 * G.bplane, SL::DEV, &bar[st]);
@@ -612,6 +605,7 @@ __global__ void __launch_bounds__(N * N, (N == 16 ? 3 : 8)) k_mp_collide(const _
             }
         }
         collide_store<N, FMT, READ_PU, BGK>(s, G, n, x, y, T, h, g, wr);
+        fence_proxy_async();  // the ring's writes on the stage's tile
         __syncthreads();  // the stage is read before it is refilled
         k = kn;
         st ^= 1;
@@ -877,8 +871,6 @@ __global__ void __launch_bounds__(N * N, (N == 16 ? 3 : 8))
     auto issue = [&](int st, int kk, int nn) {
         unsigned char* S = stages + st * SL::BYTES;
         if (t == 0) {
-            fence_proxy_async_all();
-            fence_proxy_async();
             mbar_expect_tx(&bar[st], 2 * SL::REST + SL::PLAN + SL::FRN);
             bulk_g2s(S + SL::O_RH, m.A1h + (size_t)nn * AP, SL::REST, &bar[st]);
             bulk_g2s(S + SL::O_RG, m.A1g + (size_t)nn * AP, SL::REST, &bar[st]);
