@@ -32,6 +32,8 @@ __global__ void __launch_bounds__(NT, 2)
     ConvSmem& S = *reinterpret_cast<ConvSmem*>(smraw);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, g = lane >> 2, q = lane & 3;
     load_weights(net, S, t);
+    grid_wait();
+    grid_release();
     const unsigned zero_row = smem_addr(S.zero);
     const bool explicit_ids = ids != nullptr;
     const int total = explicit_ids ? n_ids : s.cnt->nleaf;
@@ -153,7 +155,7 @@ void forecast_launch(const DevState& s, const LaunchCfg& lc, cudaStream_t st, co
     cudaFuncSetAttribute(k_forecast<MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     int grid = 2 * lc.num_sms;
     if (ids && n_ids < grid) grid = n_ids > 0 ? n_ids : 1;
-    k_forecast<MP><<<grid, NT, sm, st>>>(s, net, n_ids, ids, logits, horizon, tol, thr);
+    launch_dep(k_forecast<MP>, grid, NT, sm, st, s, net, n_ids, ids, logits, horizon, tol, thr);
 }
 
 }  // namespace

@@ -159,6 +159,8 @@ __device__ __forceinline__ bool deref_ok(const DevState& s, int n, int dir, int 
 // derefine in ascending id order (Derefine, :198-211).
 __global__ void __launch_bounds__(AMR_NTHREADS_TOPO) k_regrid_flags(DevState s, double refin_tol,
                                                                     double deref_tol) {
+    grid_wait();
+    grid_release();
     const int nb = s.cnt->nblks;
     const int lmin = s.cnt->level_min, lmax = s.cnt->level_max;
     // levels that hold a block flagged for refinement / derefinement: the
@@ -247,6 +249,8 @@ __global__ void __launch_bounds__(AMR_NTHREADS_TOPO) k_regrid_flags(DevState s, 
 // Restrict_Bilinear (Restrict.f90:14-65) for every block in der_list: the
 // parent gets the 2x2 means of its children; ghost rings are zeroed.
 __global__ void k_restrict(DevState s) {
+    grid_wait();
+    grid_release();
     const int nd = s.cnt->n_der, nx = s.nx, ny = s.ny;
     for (int i = blockIdx.x; i < nd; i += gridDim.x) {
         const int par = s.der_list[i];
@@ -362,6 +366,8 @@ __device__ void find_neighbors(const DevState& s, int par, int n, int I, int J) 
 // neighbour table of the new leaves.
 __global__ void __launch_bounds__(AMR_NTHREADS_TOPO) k_regrid_topo(DevState s, int mode, int lmin_o,
                                                                    int lmax_o, int set_levels) {
+    grid_wait();
+    grid_release();
     __shared__ int s_nr;
     Counters* cnt = s.cnt;
     const int nblks0 = cnt->nblks;
@@ -539,6 +545,8 @@ __global__ void __launch_bounds__(AMR_NTHREADS_TOPO) k_regrid_topo(DevState s, i
 // every refined block: children get bilinear h, g (with edge extrapolation)
 // and C (ring 1 included), zero ghost rings, then Macroscopic_Values_g_AMR.
 __global__ void __launch_bounds__(256) k_prolong(DevState s) {
+    grid_wait();
+    grid_release();
     extern __shared__ double T[];
     const int nr = s.cnt->n_ref, nx = s.nx, ny = s.ny, TW = nx + 4;
     for (int i = blockIdx.x; i < nr; i += gridDim.x) {
@@ -826,23 +834,23 @@ void launch_init_fields(const DevState& s, const LaunchCfg& lc, cudaStream_t st,
 }
 
 void launch_regrid_flags(const DevState& s, cudaStream_t st, double refin_tol, double deref_tol) {
-    k_regrid_flags<<<1, AMR_NTHREADS_TOPO, 0, st>>>(s, refin_tol, deref_tol);
+    launch_dep(k_regrid_flags, 1, AMR_NTHREADS_TOPO, 0, st, s, refin_tol, deref_tol);
     count_launches(1);
 }
 
 void launch_restrict(const DevState& s, const LaunchCfg& lc, cudaStream_t st) {
-    k_restrict<<<lc.grid_leaves, block_threads(s), 0, st>>>(s);
+    launch_dep(k_restrict, lc.grid_leaves, block_threads(s), 0, st, s);
     count_launches(1);
 }
 
 void launch_regrid_topo(const DevState& s, cudaStream_t st, int mode, int lmin, int lmax,
                         int set_levels) {
-    k_regrid_topo<<<1, AMR_NTHREADS_TOPO, 0, st>>>(s, mode, lmin, lmax, set_levels);
+    launch_dep(k_regrid_topo, 1, AMR_NTHREADS_TOPO, 0, st, s, mode, lmin, lmax, set_levels);
     count_launches(1);
 }
 
 void launch_prolong(const DevState& s, const LaunchCfg& lc, cudaStream_t st) {
-    k_prolong<<<lc.grid_leaves, block_threads(s), tile_bytes(s), st>>>(s);
+    launch_dep(k_prolong, lc.grid_leaves, block_threads(s), tile_bytes(s), st, s);
     count_launches(1);
 }
 

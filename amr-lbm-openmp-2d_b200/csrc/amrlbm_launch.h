@@ -13,6 +13,24 @@ enum FillCConsumer {
     CONS_MACRO_G = 3        // + Macroscopic_Values_g_AMR + Err_Interface
 };
 
+// Launch with programmatic stream serialization: the grid may become resident
+// while the one before it in the stream still runs, and holds at its
+// grid_wait() until that one has completed with its writes visible.
+template <class K, class... A>
+inline void launch_dep(K kernel, int grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, args...);
+}
+
 struct LaunchCfg {
     int num_sms;
     int grid_queue;     // CTAs of a level-ordered kernel

@@ -507,6 +507,7 @@ __device__ __forceinline__ void collide_store(const DevState& s, const Geo<N>& G
 
 template <int N, int FMT, bool READ_PU, bool BGK>
 __global__ void __launch_bounds__(N * N, (N == 16 ? 3 : 8)) k_mp_collide(const __grid_constant__ DevState s, int wr) {
+    grid_wait();
     using SL = K1Stage<N>;
     extern __shared__ __align__(128) unsigned char sm[];
     const Geo<N> G(s);
@@ -569,6 +570,7 @@ __global__ void __launch_bounds__(N * N, (N == 16 ? 3 : 8)) k_mp_collide(const _
     int st = 0;
     while (k < total) {
         const int kn = k + gridDim.x;
+        if (total <= (int)gridDim.x) grid_release();  // one item per CTA at most, as k_fill_c
         if (kn < total) item_rec_stage_async(s, kn, Q_FILLC, rec[st ^ 1]);
         if (__syncthreads_or(mbar_wait(&bar[st], (phase >> st) & 1u) ? 0 : 1)) {
             if (t == 0) set_error(s, 8 /*AMRLBM_ERR_TIMEOUT*/, 110);
@@ -829,6 +831,7 @@ __device__ void hg_item(const DevState& s, const Geo<N>& G, int k, const ItemRec
 template <int N, int FMT>
 __global__ void __launch_bounds__(N * N, (N == 16 ? 3 : 8))
     k_mp_fill_hg_stream(const __grid_constant__ DevState s, int wr) {
+    grid_wait();
     using SL = K2Stage<N>;
     constexpr int AP = SL::AP, FP = 9 * AP;
     extern __shared__ __align__(128) unsigned char sm[];
@@ -902,6 +905,7 @@ __global__ void __launch_bounds__(N * N, (N == 16 ? 3 : 8))
     int st = 0;
     while (k < total) {
         const int kn = k + gridDim.x;
+        if (total <= (int)gridDim.x) grid_release();  // one item per CTA at most, as k_fill_c
         if (kn < total) issue(st ^ 1, kn, s_nn);
         else cp_async_commit();  // an empty group keeps the wait count uniform
         if (t == 0 && kn + (int)gridDim.x < total) n_after = __ldg(s.lvl_leaf + kn + gridDim.x);
@@ -945,6 +949,7 @@ __global__ void __launch_bounds__(N * N, (N == 16 ? 3 : 8))
 // Err_Interface (Refine_Derefine.f90:327-351, into the FP64 err of the block)
 template <int N, int FMT>
 __global__ void __launch_bounds__(N * N) k_mp_tail(const __grid_constant__ DevState s) {
+    grid_wait();
     const Geo<N> G(s);
     __shared__ float T[cplane_of(N)];
     extern __shared__ float Fs[];
@@ -1014,6 +1019,7 @@ __device__ __forceinline__ int conv_block(const DevState& s, int mode, int i) {
 template <int N, int FMT>
 __global__ void __launch_bounds__(256) k_mp_convert(const __grid_constant__ DevState s, int mode,
                                                     int to_mp) {
+    grid_wait();
     const Geo<N> G(s);
     const MpState& m = s.mp;
     const int cnt = conv_count(s, mode);
@@ -1132,7 +1138,7 @@ void grid_leaves_launch(K kern, const LaunchCfg& lc, int threads, size_t dyn, cu
     int b = per_sm(kern, threads, dyn);
     if (prepare) return;
     if (lc.mp_ctas > 0 && lc.mp_ctas < b) b = lc.mp_ctas;
-    kern<<<lc.num_sms * b, threads, dyn, st>>>(s, a);
+    launch_dep(kern, lc.num_sms * b, threads, dyn, st, s, a);
     count_launches(1);
 }
 
@@ -1162,12 +1168,12 @@ void mp_fill_hg(const DevState& s, const LaunchCfg& lc, cudaStream_t st, int wr,
 }
 template <int N, int FMT>
 void mp_tail(const DevState& s, const LaunchCfg& lc, cudaStream_t st) {
-    k_mp_tail<N, FMT><<<lc.grid_leaves, N * N, sizeof(float) * (size_t)s.fmax, st>>>(s);
+    launch_dep(k_mp_tail<N, FMT>, lc.grid_leaves, N * N, sizeof(float) * (size_t)s.fmax, st, s);
     count_launches(1);
 }
 template <int N, int FMT>
 void mp_convert(const DevState& s, const LaunchCfg& lc, cudaStream_t st, int mode, int to_mp) {
-    k_mp_convert<N, FMT><<<lc.grid_leaves, 256, 0, st>>>(s, mode, to_mp);
+    launch_dep(k_mp_convert<N, FMT>, lc.grid_leaves, 256, 0, st, s, mode, to_mp);
     count_launches(1);
 }
 
