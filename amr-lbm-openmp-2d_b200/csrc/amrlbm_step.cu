@@ -24,6 +24,7 @@
 #include "amrlbm_fast.cuh"
 #include "amrlbm_launch.h"
 #include "amrlbm_plan.cuh"
+#include "amrlbm_wait.h"
 
 void count_launches(int n);
 
@@ -1529,10 +1530,10 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, const Geo
     unsigned long long* bar = S.bar;
     double *As = S.As, *Fs = S.Fs;
     int* Ps = S.Ps;
-    unsigned phase = 0;  // bit b: parity of bar[b]'s next completion
 
     if (FAST) {
         __shared__ int srec[2][REC_WORDS];  // records of the current and the next item
+        unsigned phase = 0;  // bit b: parity of bar[b]'s next completion
         int c = blockIdx.x, rb = 0;
         if (c < total) item_rec_stage(s, c, q, srec[0]);
         __syncthreads();
@@ -1588,10 +1589,21 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, const Geo
     }
 
     __syncthreads();  // the mbarriers are initialised
-    // the copies issued at entry land before anything else uses the stage
-    const bool landed = mbar_wait(&bar[0], 0) && mbar_wait(&bar[1], 0);
-    if (!landed && t == 0) set_error(s, 8 /*AMRLBM_ERR_TIMEOUT*/, 100 + q);
-    phase = 3u;
+    CopyWaits cw;
+    auto landed = [&](unsigned bits) {
+        const bool ok = cw.landed(
+            bits, bits, [&](int b, unsigned p) { return mbar_wait(&bar[b], p); },
+            [](bool late) { return __syncthreads_or(late) != 0; });
+        if (!ok && t == 0) set_error(s, 8 /*AMRLBM_ERR_TIMEOUT*/, 100 + q);
+        return ok;
+    };
+    // The copies issued at entry land before anything else uses the stage. A
+    // CTA whose copies do not leaves, and the others take its share of the
+    // queues, of which it has claimed nothing yet.
+    if (!landed(3u)) {
+        queue_done(s, q);
+        return;
+    }
     const int lmin = s.cnt->level_min;
     fill_phase(
         s, q, nbis, &s_next,
@@ -1620,12 +1632,7 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, const Geo
             S.copy_planes(n);
             s_next = (int)cn;
         }
-        if (__syncthreads_or(mbar_wait(bar, phase & 1u) ? 0 : 1)) {
-            if (t == 0) set_error(s, 8 /*AMRLBM_ERR_TIMEOUT*/, 100 + q);
-            mbar_wait(bar, phase & 1u);
-            break;
-        }
-        phase ^= 1u;
+        if (!landed(1u)) break;
         stream_block<N>(s, G, n, As, StreamCoef(__ldg(s.dx + n)));
         c = s_next;
         __syncthreads();
