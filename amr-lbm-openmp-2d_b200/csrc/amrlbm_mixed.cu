@@ -28,6 +28,7 @@
 #include "amrlbm_fast.cuh"
 #include "amrlbm_launch.h"
 #include "amrlbm_plan.cuh"
+#include "amrlbm_wait.h"
 
 void count_launches(int n);
 
@@ -901,7 +902,7 @@ __global__ void __launch_bounds__(N * N, (N == 16 ? 3 : 8))
     __syncthreads();
     if (t == 0) s_nn = n_after;
     __syncthreads();
-    unsigned phase = 0;
+    CopyWaits cw;
     int st = 0;
     while (k < total) {
         const int kn = k + gridDim.x;
@@ -910,13 +911,14 @@ __global__ void __launch_bounds__(N * N, (N == 16 ? 3 : 8))
         else cp_async_commit();  // an empty group keeps the wait count uniform
         if (t == 0 && kn + (int)gridDim.x < total) n_after = __ldg(s.lvl_leaf + kn + gridDim.x);
         cp_async_wait_prev();
-        if (__syncthreads_or(mbar_wait(&bar[st], (phase >> st) & 1u) ? 0 : 1)) {
+        // (the next item's copies are in flight already)
+        if (!cw.landed(
+                st, kn < total ? 3u : 1u << st,
+                [&](int b, unsigned p) { return mbar_wait(&bar[b], p); },
+                [](bool late) { return __syncthreads_or(late) != 0; })) {
             if (t == 0) set_error(s, 8 /*AMRLBM_ERR_TIMEOUT*/, 111);
-            mbar_wait(&bar[st], (phase >> st) & 1u);
-            cp_async_wait_all();
             break;
         }
-        phase ^= 1u << st;
         const unsigned char* S = stages + st * SL::BYTES;
         const ItemRec r = item_rec_of(rec[st]);
         // decode the staged planes into As

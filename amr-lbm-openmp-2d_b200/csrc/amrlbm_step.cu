@@ -1590,9 +1590,9 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, const Geo
 
     __syncthreads();  // the mbarriers are initialised
     CopyWaits cw;
-    auto landed = [&](unsigned bits) {
+    auto landed = [&](int b, unsigned in_flight) {
         const bool ok = cw.landed(
-            bits, bits, [&](int b, unsigned p) { return mbar_wait(&bar[b], p); },
+            b, in_flight, [&](int i, unsigned p) { return mbar_wait(&bar[i], p); },
             [](bool late) { return __syncthreads_or(late) != 0; });
         if (!ok && t == 0) set_error(s, 8 /*AMRLBM_ERR_TIMEOUT*/, 100 + q);
         return ok;
@@ -1600,7 +1600,7 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, const Geo
     // The copies issued at entry land before anything else uses the stage. A
     // CTA whose copies do not leaves, and the others take its share of the
     // queues, of which it has claimed nothing yet.
-    if (!landed(3u)) {
+    if (!landed(0, 3u) || !landed(1, 2u)) {
         queue_done(s, q);
         return;
     }
@@ -1632,7 +1632,7 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, const Geo
             S.copy_planes(n);
             s_next = (int)cn;
         }
-        if (!landed(1u)) break;
+        if (!landed(0, 1u)) break;
         stream_block<N>(s, G, n, As, StreamCoef(__ldg(s.dx + n)));
         c = s_next;
         __syncthreads();

@@ -15,23 +15,20 @@
 struct CopyWaits {
     unsigned parity = 0;  // bit b: parity of barrier b's next completion
 
-    // Bounded waits for the barriers of mask `wait`. wait_on(b, parity): whether
-    // barrier b completed in time; any(x): x of some thread of the CTA. Every
-    // thread gets the same answer. On false every thread has waited (bounded)
-    // once more for all the barriers of mask `in_flight`, so that no copy writes
-    // into shared memory that the CTA has given up, and the caller leaves
-    // without using what did not land.
+    // Bounded wait for barrier b. wait_on(b, parity): whether barrier b completed
+    // in time; any(x): x of some thread of the CTA. Every thread gets the same
+    // answer. On false every thread has waited (bounded) once more for all the
+    // barriers of mask `in_flight`, so that no copy writes into shared memory
+    // that the CTA has given up, and the caller leaves without using what did
+    // not land.
     template <class WAIT, class ANY>
-    AMR_WAIT_FN bool landed(unsigned wait, unsigned in_flight, WAIT wait_on, ANY any) {
-        bool late = false;
-        for (int b = 0; b < 2; ++b)
-            if ((wait >> b) & 1u) late |= !wait_on(b, (parity >> b) & 1u);
-        if (any(late)) {
-            for (int b = 0; b < 2; ++b)
-                if ((in_flight >> b) & 1u) wait_on(b, (parity >> b) & 1u);
+    AMR_WAIT_FN bool landed(int b, unsigned in_flight, WAIT wait_on, ANY any) {
+        if (any(!wait_on(b, (parity >> b) & 1u))) {
+            for (int i = 0; in_flight >> i; ++i)
+                if ((in_flight >> i) & 1u) wait_on(i, (parity >> i) & 1u);
             return false;
         }
-        parity ^= wait;
+        parity ^= 1u << b;
         return true;
     }
 };

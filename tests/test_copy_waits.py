@@ -25,10 +25,10 @@ struct Barrier {
 };
 int main(int, char** v) {
     Barrier bar[2] = {{atoi(v[1])}, {atoi(v[2])}};
-    const unsigned wait = atoi(v[3]), in_flight = atoi(v[4]);
+    const int b = atoi(v[3]);
     CopyWaits w;
     auto on = [&](int b, unsigned p) { return bar[b].wait(p); };
-    const bool ok = w.landed(wait, in_flight, on, [](bool x) { return x; });
+    const bool ok = w.landed(b, atoi(v[4]), on, [](bool x) { return x; });
     printf("%d %u %d %d\n", ok, w.parity, bar[0].waits, bar[1].waits);
 }
 """
@@ -44,17 +44,20 @@ def program(tmp_path_factory):
 
 
 @pytest.mark.parametrize("lands,wait,in_flight,want", [
-    # in time: one wait each, the parities of the awaited barriers advance
-    ((0, 0), 3, 3, (1, 3, 1, 1)),
-    ((0, 0), 1, 3, (1, 1, 1, 0)),
-    ((0, -1), 1, 3, (1, 1, 1, 0)),
-    # one of two late: the caller must not go on, whichever it is, and both
-    # have been waited for again
-    ((1, 0), 3, 3, (0, 0, 2, 2)),
-    ((0, 1), 3, 3, (0, 0, 2, 2)),
-    # never: parity stays, or the next wait would pass at once
-    ((-1, -1), 3, 3, (0, 0, 2, 2)),
-    ((-1, 0), 1, 1, (0, 0, 2, 0)),
+    # in time: one wait, the awaited barrier's parity advances
+    ((0, 0), 0, 3, (1, 1, 1, 0)),
+    ((0, -1), 0, 1, (1, 1, 1, 0)),
+    ((-1, 0), 1, 2, (1, 2, 0, 1)),
+    # late: the caller must not go on, though the copy has landed by now
+    ((1, 0), 0, 1, (0, 0, 2, 0)),
+    ((0, 1), 1, 2, (0, 0, 0, 2)),
+    # never: the parity stays, or the next wait would pass at once
+    ((-1, -1), 0, 1, (0, 0, 2, 0)),
+    # the copies behind the other barrier are waited for too, where some are
+    # in flight
+    ((-1, 0), 0, 3, (0, 0, 2, 1)),
+    ((1, -1), 0, 3, (0, 0, 2, 1)),
+    ((0, -1), 1, 3, (0, 0, 1, 2)),
 ])
 def test_late_copies(program, lands, wait, in_flight, want):
     out = subprocess.run([program, *map(str, (*lands, wait, in_flight))], check=True,
