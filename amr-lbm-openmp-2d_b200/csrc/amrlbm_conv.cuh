@@ -122,7 +122,8 @@ __device__ __forceinline__ void ldsm4(unsigned addr, unsigned& r0, unsigned& r1,
 // channels, so the operand fragments come by ldmatrix: A rows are the
 // activation rows of the shifted pixels (a zero row outside the tile), B the
 // transposed weights. The warp's row tiles mt = warp, warp + 8, warp + 16
-// share each step's B fragments. Accumulation order along K as k_gemm's.
+// share each step's B fragments. Accumulated along K from the first column on,
+// 16 at a time.
 template <int KW>
 __device__ __forceinline__ void conv32(const __nv_bfloat16 (*act)[AROW], const __nv_bfloat16 (*wt)[KW],
                                        unsigned zero_row, int warp, int lane, float acc[3][4][4]) {

@@ -14,6 +14,8 @@
 // Programmatic dependent launch. grid_wait: until the grid before this one has
 // completed and its writes are visible (at once where it was launched
 // without); every thread passes it before it reads what that grid may write.
+// What is read before it (k_fill_hg_stream's leaf count, plans and foreign
+// records, the forecaster's weights) only earlier grids write, or none.
 // Earlier grids have completed before it: that grid, too, released its
 // dependents only after its own wait. grid_release: the next grid may become
 // resident; never before grid_wait, and implied when a CTA exits. A step's

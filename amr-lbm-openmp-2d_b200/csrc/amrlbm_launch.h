@@ -44,6 +44,8 @@ struct LaunchCfg {
 // CONS_NONE always write them
 void launch_fill_c(const DevState& s, const LaunchCfg& lc, cudaStream_t st, int width,
                    int consumer, int write_ring = 1);
+// (a collision must be the launch before it: the kernel reads the leaf count and
+// the plans before it waits for that grid)
 void launch_fill_hg_stream(const DevState& s, const LaunchCfg& lc, cudaStream_t st,
                            int write_ring = 1);
 void launch_collide(const DevState& s, const LaunchCfg& lc, cudaStream_t st);

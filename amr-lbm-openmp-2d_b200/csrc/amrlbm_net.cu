@@ -36,7 +36,8 @@ constexpr int O_W1 = 0, O_B1 = O_W1 + K1 * CH, O_W2 = O_B1 + CH, O_B2 = O_W2 + K
               O_W3 = O_B2 + CH, O_B3 = O_W3 + K2 * CH, O_WD = O_B3 + CH, O_BD = O_WD + CH,
               NPARAM = O_BD + 1;
 
-// ---- the tensor-core product -----------------------------------------------
+// ---- the plain tensor-core product, for amrlbm_net_selftest_gemm alone ---------
+// (the network's own products are those of k_net and k_dw)
 // C[M][N] (FP32, row stride ldc) = sum_k A(m, k) B(k, n), A(m, k) = A[m*sam + k*sak],
 // B(k, n) = B[k*sbk + n*sbn], BF16. CTA: 4 warps, a 64 x 32 tile of C; each
 // warp 16 rows x 4 n-tiles of 8. Operands go through shared memory with zero
@@ -214,10 +215,11 @@ __device__ __forceinline__ void conv32_back(const __nv_bfloat16 (*dz)[AROW], con
 // The gradients equal, bit for bit, those of the plain sequence of products and
 // elementwise kernels that this replaced (im2col, product, bias and ReLU;
 // backwards product, col2im): the same operands in the same order.
-// What bounds it: some 5,000 mma.sync per sample with the ldmatrix that feed
-// them, 8 warps per CTA; one CTA per SM for the gradient (175 KB of shared
-// memory), two for the forward pass. The im2col matrices of that sequence,
-// 191 MB per layer for 512 samples, took 1.7 ms per gradient.
+// What bounds it: the mma.sync of a sample (3,276 forward, 6,300 with the
+// gradient) and the ldmatrix that feed them, 8 warps per CTA; one CTA per SM
+// for the gradient (175 KB of shared memory), two for the forward pass. The
+// im2col matrices of that sequence, 191 MB per layer for 512 samples, took
+// 1.7 ms per gradient.
 template <bool GRAD>
 __global__ void __launch_bounds__(NT, GRAD ? 1 : 2)
     k_net(const ForecastNet net, int n, const float* x, const float* y, float posw, float* logits,

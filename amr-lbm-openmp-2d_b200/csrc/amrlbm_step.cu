@@ -612,12 +612,12 @@ __device__ void wall_c(const DevState& s, const Geo<N>& G, int n, const NbInfo& 
 }
 
 // ---------------------------------------------------------------------------
-// Collision_h_g_AMR (LBM_Subroutines.f90:116-189) of cell c of block n.
-// with IEEE divisions. T: shared C block (G.c(0,..)); the post-streaming h and
-// g planes are read from memory; unless FUSED, P, Ux, Uy are read from memory, where nothing writes them during the
-// launch. Writes the post-collision populations A to memory. FUSED: P, Ux,
-// Uy come from Macroscopic_Values_g_AMR (:205-240) evaluated here on the
-// same C ring.
+// Collision_h_g_AMR (LBM_Subroutines.f90:116-189) of cell c of block n, with
+// IEEE divisions. T: shared C block (G.c(0,..)). The post-streaming h and g
+// planes are read from memory; so are P, Ux, Uy unless FUSED (nothing writes
+// them during the launch). Writes the post-collision populations A to memory.
+// FUSED: P, Ux, Uy come from Macroscopic_Values_g_AMR (:205-240) evaluated
+// here on the same C ring.
 // BGK: the collision of g is BGK_Collision_AMR (LBM_Subroutines.f90:337-344,
 // g*(1-s9) + geq*s9) instead of MRT_Collision_AMR, the alternative the
 // reference leaves commented out at :180
@@ -747,8 +747,10 @@ __device__ __forceinline__ void collide_ieee(const DevState& s, const Geo<N>& G,
     }
 }
 
-// The same collision, bit for bit (up to the sign of zeros), with about three
-// quarters of the FP64 operations: opposite directions share their terms
+// The same collision with about three quarters of the FP64 operations, bit for
+// bit up to the sign of zeros and except where differences of C lie below
+// 2^-1000 (there 1/dx times them is no longer exact, and the reference's
+// rounding is carried to within 2^-1070): opposite directions share their terms
 // (Ec(-e) = -Ec(e), 4.5 eU, eU (3 +- 4.5 eU)), products by powers of two (0.5,
 // 2, 4, 1/dx) ride in exact FMAs, gradients are formed unscaled and scaled
 // once (1/dx is a power of two), and zero components of e drop out. Where that
@@ -756,9 +758,7 @@ __device__ __forceinline__ void collide_ieee(const DevState& s, const Geo<N>& G,
 // is returned and the caller takes collide_ieee, which reads h and g from
 // memory. SMEM: the block's h and g planes Hb, Gb are staged in shared memory,
 // and each population h of this cell, once read, gives its place to hm (the
-// forcing of g), which is needed only at the end. Differences of C below
-// 2^-1000, where 1/dx times them is no longer exact, carry the reference's
-// rounding to within 2^-1070.
+// forcing of g), which is needed only at the end.
 // The consumer shares the CTA's time with the copies and the ghost fill, so
 // fewer operations gave 26.0 -> 25.4 us over 788 leaves of 16x16 cells and
 // 455 -> 450 us over 17,568; three CTAs per SM (80 registers, one stage) were
@@ -1445,8 +1445,9 @@ __device__ __forceinline__ void fill_c_body(const DevState& s, int w, int q, int
         __syncwarp();  // warp 0 reconverges after thread 0's copies, before the consumer work
         // One item per CTA at most: the next grid's CTAs may come in beside it.
         // With more, those would take their places (and this grid's split of
-        // L1 and shared memory) while it still has items: 46.4 us per step
-        // against 39.6 (788 leaves), 945 against 795 (17,568)
+        // L1 and shared memory) while it still has items: with a release at the
+        // entry of every kernel a step took 46.4 us instead of 40.3 (788
+        // leaves) and 945 instead of 799 (17,568)
         if (fast && total <= (int)gridDim.x) grid_release();
         consume(n, fast ? r.dx : __ldg(s.dx + n), T);
         if (fast) cp_async_wait_all();  // the next item's record
@@ -1644,6 +1645,12 @@ __device__ __forceinline__ void fill_hg_stream_body(const DevState& s, const Geo
 // the fill needs level order, so its plan, then its planes, are copied at
 // entry, before the flags that tell which path runs arrive (the pools hold
 // max_blks + 1 blocks and plans: any index the work order holds is in range).
+// The leaf count, the plan and the foreign records are read before grid_wait:
+// the grid directly before this one in the stream must write none of them (not
+// k_regrid_topo or k_build_plans; grids before that one have completed). Every
+// launch follows a collision (k_fill_c, k_collide). Reading them behind the wait
+// made a step about 1 % longer (small bubble, a regrid each: 40.7 -> 41.0 us;
+// 12x10 blocks: 34.8 -> 35.2 us).
 template <int N>
 __global__ void __launch_bounds__(256, 3)
     k_fill_hg_stream(const __grid_constant__ DevState s, int wr) {

@@ -349,8 +349,9 @@ int amrlbm_net_train_step(amrlbm_net* net, int32_t n, const float* x, const floa
                           float pos_weight, float lr, float* loss);
 /* logits of n samples already in device memory (any n) */
 int amrlbm_net_forward_device(amrlbm_net* net, int32_t n, const float* x_dev, float* logits);
-/* the network's tensor-core product alone: C = A B, A [M][K] and B [K][N]
- * BF16 bit patterns, C FP32, row-major host arrays */
+/* a plain tensor-core product (mma.sync m16n8k16, as the network's, but not on
+ * its path): C = A B, A [M][K] and B [K][N] BF16 bit patterns, C FP32, row-major
+ * host arrays */
 int amrlbm_net_selftest_gemm(int32_t M, int32_t N, int32_t K, const uint16_t* A,
                              const uint16_t* B, float* C);
 
