@@ -145,8 +145,8 @@ int amrlbm_set_launch(amrlbm_ctx* ctx, int32_t ctas_per_sm);
  * A fill needs it where a coarse-to-fine stencil reads a coarser
  * neighbour's ghost cell that is itself coarse-to-fine, or one behind a wall
  * beside such a cell (the reference's DO L = LevelMin, LevelMax loops,
- * Fill_Ghost_Cells_C.f90:8-38);
- * its kernels then take the leaves in level order with bounded waits. A
+ * Fill_Ghost_Cells_C.f90:8-38); its kernels then take the leaves in level
+ * order with bounded waits. None does on a mesh within the 2:1 balance. A
  * performance diagnostic; no counterpart in the reference. */
 int amrlbm_get_fill_order(amrlbm_ctx* ctx, int32_t needs_order[3]);
 /* Failure-detection test hook; no counterpart in the reference, whose
